@@ -33,11 +33,28 @@ constexpr int kEmpty = 0x7FFFFFFF;  // "stack exhausted"
 #endif
 constexpr uint32_t kRefill = GBRT_REFILL;  // idle lanes that trigger a refill
 
+// Rays a warp takes from the queue at a time.  A queue of few rays is spread
+// over half of the launch's warps instead of filling the first ones: a warp's
+// time grows with the rays whose ways through the tree it serialises, and the
+// other warps would idle.  Frames of one sample at depth 8, us of device time
+// with 32 / 8 / 4 / 2 / 1 rays at least (all of the warps: half): 64 x 64
+// Cornell 214 / 185 / 184 / 183 / 204, 128 x 128 instanced tori 1636 / 1402 /
+// 1310 / 1255 / 1198; half of the warps instead of all: 512 x 256 icosphere 626
+// against 659, 128 x 128 tori 1338 against 1310.
+#ifndef GBRT_MIN_QUOTA
+#define GBRT_MIN_QUOTA 2
+#endif
+constexpr uint32_t kMinQuota = GBRT_MIN_QUOTA;
+GB_D uint32_t ray_quota(uint32_t n, uint32_t warps) {
+    const unsigned long long q = (2ull * n + warps - 1u) / warps;
+    return q < kMinQuota ? kMinQuota : (q < 32u ? (uint32_t)q : 32u);
+}
+
 // Loader: bool load(uint32_t q, float3& o, float3& d, float& tmin, float& tmax, AnyCtx& ctx)
 // Finisher: void finish(uint32_t q, bool hit, const Hit& h)
 template <bool kAny, bool kAlpha, class Loader, class Finisher>
 GB_D void persistent_trace(const DevScene& s, uint32_t n, uint32_t* work, uint32_t flags, TraceStats& ts,
-                           Loader&& load, Finisher&& finish) {
+                           uint32_t quota, Loader&& load, Finisher&& finish) {
     const uint32_t lane = threadIdx.x & 31u;
     const bool test_alpha = kAlpha && !(flags & GBRT_RAY_OPAQUE) && !s.all_opaque;
     int stack_node[kStack];
@@ -55,12 +72,14 @@ GB_D void persistent_trace(const DevScene& s, uint32_t n, uint32_t* work, uint32
         if (!exhausted) {
             const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !has);
             if (__popc(idle) >= (int)kRefill) {
+                const uint32_t take = min((uint32_t)__popc(idle), quota);
                 uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(work, (uint32_t)__popc(idle));
+                if (lane == 0) base = atomicAdd(work, take);
                 base = __shfl_sync(0xFFFFFFFFu, base, 0);
-                if (base + __popc(idle) >= n) exhausted = true;
-                if (!has) {
-                    q = base + __popc(idle & ((1u << lane) - 1u));
+                if (base + take >= n) exhausted = true;
+                const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
+                if (!has && rank < take) {
+                    q = base + rank;
                     if (q < n) {
                         float3 o, d;
                         load(q, o, d, tmin, tmax, ctx);
@@ -203,7 +222,7 @@ namespace gbrt {
 // refill policy as persistent_trace.
 template <bool kAny, bool kTlas, bool kAlpha, class Loader, class Finisher>
 GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uint32_t flags, TraceStats& ts,
-                              Loader&& load, Finisher&& finish) {
+                              uint32_t quota, Loader&& load, Finisher&& finish) {
     const uint32_t lane = threadIdx.x & 31u;
     const bool test_alpha = kAlpha && !(flags & GBRT_RAY_OPAQUE) && !s.all_opaque;
 #if GBRT_CW_SMEM_STACK
@@ -237,12 +256,14 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
         if (!exhausted) {
             const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !has);
             if (__popc(idle) >= (int)kRefill) {
+                const uint32_t take = min((uint32_t)__popc(idle), quota);
                 uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(work, (uint32_t)__popc(idle));
+                if (lane == 0) base = atomicAdd(work, take);
                 base = __shfl_sync(0xFFFFFFFFu, base, 0);
-                if (base + __popc(idle) >= n) exhausted = true;
-                if (!has) {
-                    q = base + __popc(idle & ((1u << lane) - 1u));
+                if (base + take >= n) exhausted = true;
+                const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
+                if (!has && rank < take) {
+                    q = base + rank;
                     if (q < n) {
                         float3 o, d;
                         load(q, o, d, tmin, tmax, ctx);
@@ -352,12 +373,28 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
 constexpr int kTraceBinary = 0, kTraceWide = 1, kTraceWideTlas = 2, kTraceOpaque = 4;
 
 template <bool kAny, int kMode, class Loader, class Finisher>
-GB_D void world_trace(const DevScene& s, uint32_t n, uint32_t* work, uint32_t flags, TraceStats& ts, Loader&& load,
-                      Finisher&& finish) {
+GB_D void world_trace(const DevScene& s, uint32_t n, uint32_t* work, uint32_t flags, TraceStats& ts,
+                      uint32_t warps, Loader&& load, Finisher&& finish) {
     constexpr int kForm = kMode & 3;
     constexpr bool kAlpha = !(kMode & kTraceOpaque);
-    if constexpr (kForm == kTraceBinary) persistent_trace<kAny, kAlpha>(s, n, work, flags, ts, load, finish);
-    else persistent_trace_cw<kAny, kForm == kTraceWideTlas, kAlpha>(s, n, work, flags, ts, load, finish);
+    const uint32_t quota = ray_quota(n, warps);
+    if constexpr (kForm == kTraceBinary) persistent_trace<kAny, kAlpha>(s, n, work, flags, ts, quota, load, finish);
+    else persistent_trace_cw<kAny, kForm == kTraceWideTlas, kAlpha>(s, n, work, flags, ts, quota, load, finish);
+}
+
+// Launch shape of a traversal kernel over at most n rays, `resident` blocks
+// of 128 threads filling the GPU: full blocks when every resident warp gets
+// rays, else one-warp blocks, one per kMinQuota rays, which spread over all
+// SMs and leave no warp that only finds its queue empty.  The 64 x 64 Cornell
+// frame takes 246 us instead of 284 with the quota, these grids, the shade
+// blocks of shade_threads and queue_done.
+struct TraceGrid {
+    uint32_t blocks, threads;
+};
+inline TraceGrid trace_grid(int resident, uint64_t n) {
+    const uint64_t full = (uint64_t)resident * 4, warps = (n + kMinQuota - 1) / kMinQuota;
+    if (warps >= full) return {(uint32_t)resident, 128u};
+    return {warps ? (uint32_t)warps : 1u, 32u};
 }
 
 // The form a scene needs: binary when it has a world BVH without its

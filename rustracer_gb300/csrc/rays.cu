@@ -12,7 +12,7 @@ __global__ void __launch_bounds__(128) trace_rays_persistent(DevScene s, const g
                                                              DeviceCounters* cnt) {
     TraceStats ts{0, 0, 0};
     world_trace<kAny, kMode>(
-        s, n, work, flags, ts,
+        s, n, work, flags, ts, gridDim.x * (blockDim.x >> 5),
         [&](uint32_t q, float3& o, float3& d, float& tmin, float& tmax, AnyCtx& ctx) {
             const gbrt_ray r = rays[q];
             o = f3(r.org[0], r.org[1], r.org[2]);
@@ -31,17 +31,7 @@ __global__ void __launch_bounds__(128) trace_rays_persistent(DevScene s, const g
             g.custom_index = hit ? s.inst[h.inst].custom : 0xFFFFFFFFu;
             hits[q] = g;
         });
-    if (cnt) {
-        const unsigned long long nodes = warp_sum<unsigned long long>(ts.nodes);
-        const unsigned long long tris = warp_sum<unsigned long long>(ts.tris);
-        uint32_t stat = ts.status;
-        for (int o = 16; o > 0; o >>= 1) stat |= __shfl_down_sync(0xFFFFFFFFu, stat, o);
-        if ((threadIdx.x & 31u) == 0) {
-            atomicAdd(&cnt->nodes, nodes);
-            atomicAdd(&cnt->tris, tris);
-            if (stat) atomicOr(&cnt->status, stat);
-        }
-    }
+    if (cnt) flush_trace_stats(ts, cnt);
 }
 
 cudaError_t launch_trace_rays_persistent(const DevScene& s, const gbrt_ray* rays, uint32_t n, uint32_t flags,
@@ -61,17 +51,16 @@ cudaError_t launch_trace_rays_persistent(const DevScene& s, const gbrt_ray* rays
         dev_cached = dev;
     }
     if ((e = cudaMemsetAsync(work, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-    const uint32_t need = (n + 127) / 128;
-    const uint32_t grid = need < (uint32_t)resident ? need : (uint32_t)resident;
+    const TraceGrid g = trace_grid(resident, n);
     const bool any = flags & GBRT_RAY_TERMINATE_ON_FIRST;
     // ray queries use the 8-wide form with the TLAS (it skips the TLAS of
     // scenes without one), or the binary form where the scene needs it
     if (trace_mode(s) != kTraceBinary) {
-        if (any) trace_rays_persistent<true, kTraceWideTlas><<<grid, 128, 0, st>>>(s, rays, n, flags, hits, work, cnt);
-        else trace_rays_persistent<false, kTraceWideTlas><<<grid, 128, 0, st>>>(s, rays, n, flags, hits, work, cnt);
+        if (any) trace_rays_persistent<true, kTraceWideTlas><<<g.blocks, g.threads, 0, st>>>(s, rays, n, flags, hits, work, cnt);
+        else trace_rays_persistent<false, kTraceWideTlas><<<g.blocks, g.threads, 0, st>>>(s, rays, n, flags, hits, work, cnt);
     } else {
-        if (any) trace_rays_persistent<true, kTraceBinary><<<grid, 128, 0, st>>>(s, rays, n, flags, hits, work, cnt);
-        else trace_rays_persistent<false, kTraceBinary><<<grid, 128, 0, st>>>(s, rays, n, flags, hits, work, cnt);
+        if (any) trace_rays_persistent<true, kTraceBinary><<<g.blocks, g.threads, 0, st>>>(s, rays, n, flags, hits, work, cnt);
+        else trace_rays_persistent<false, kTraceBinary><<<g.blocks, g.threads, 0, st>>>(s, rays, n, flags, hits, work, cnt);
     }
     return cudaGetLastError();
 }

@@ -214,13 +214,13 @@ cudaError_t enqueue_wave(const WfState& st, int mode, uint32_t nb, cudaStream_t 
     te();
     for (uint32_t b = 0; b < nb; ++b) {
         tb(0);
-        GBRT_TRACE_LAUNCH(wfm_extend, g_grid.extend, stream, st, b);
+        GBRT_TRACE_LAUNCH(wfm_extend, g_grid.extend, 128, stream, st, b);
         te();
         tb(1);
         wfm_shade<<<g_grid.shade, kShadeThreads, 0, stream>>>(st, b);
         te();
         tb(2);
-        GBRT_TRACE_LAUNCH(wfm_shadow, g_grid.shadow, stream, st, b);
+        GBRT_TRACE_LAUNCH(wfm_shadow, g_grid.shadow, 128, stream, st, b);
         te();
     }
     tb(3);

@@ -104,7 +104,7 @@ cudaError_t init_wavefront_constants(const float* srgb_lut) {
 namespace {
 struct Grid {
     int dev = -1;
-    int extend = 0, shade = 0, shade_plain = 0, shadow = 0;
+    int sms = 0, extend = 0, shade = 0, shade_plain = 0, shadow = 0;
 };
 Grid g_grid;
 
@@ -126,8 +126,21 @@ cudaError_t grids(Grid& g) {
     g.extend = sms * (be > 0 ? be : 1);
     g.shade = sms * (bs > 0 ? bs : 1);
     g.shadow = sms * (bh > 0 ? bh : 1);
+    g.sms = sms;
     g.dev = dev;
     return cudaSuccess;
+}
+
+// Block size of a shade kernel compiled for `full` threads over at most n
+// paths: the full size (long runs of rays grouped by octant) once n fills two
+// blocks per SM, else blocks small enough that a wave reaches every SM.
+uint32_t shade_threads(uint32_t n, uint32_t full) {
+    const uint32_t per = (n / (2u * (uint32_t)g_grid.sms) + 31u) / 32u * 32u;
+    return per < 32u ? 32u : (per < full ? per : full);
+}
+uint32_t shade_blocks(uint32_t n, uint32_t threads, int resident) {
+    const uint32_t need = (n + threads - 1u) / threads;
+    return need < (uint32_t)resident ? need : (uint32_t)resident;
 }
 }  // namespace
 
@@ -235,18 +248,22 @@ cudaError_t launch_wavefront(const DevScene& s, const gbrt_ubo& ubo, const Rende
                 if ((e = cudaMemsetAsync(nrc->snap_pos, 0, (size_t)J.npaths * sizeof(float4), stream)) != cudaSuccess)
                     return e;
             }
+            const TraceGrid ge = trace_grid(g_grid.extend, J.npaths), gh = trace_grid(g_grid.shadow, J.npaths);
+            const uint32_t ts = shade_threads(J.npaths, kShadeThreads), tp = shade_threads(J.npaths, kShadePlainThreads);
+            const uint32_t bs = shade_blocks(J.npaths, ts, g_grid.shade),
+                           bp = shade_blocks(J.npaths, tp, g_grid.shade_plain);
             tb(3);
             wf_camera<<<(J.npaths + 127) / 128, 128, 0, stream>>>(w, st);
             te();
             for (uint32_t b = 0; b < nb; ++b) {
                 tb(0);
-                GBRT_TRACE_LAUNCH(wf_extend, g_grid.extend, stream, w, st, b);
+                GBRT_TRACE_LAUNCH(wf_extend, ge.blocks, ge.threads, stream, w, st, b);
                 te();
                 if (side && b > 0 && (e = cudaStreamWaitEvent(stream, side->shadowed, 0)) != cudaSuccess) return e;
                 tb(1);
-                if (nrc) wf_shade_nrc<<<g_grid.shade, kShadeThreads, 0, stream>>>(w, st, b, *nrc);
-                else if (feat == 0u) wf_shade<0u><<<g_grid.shade_plain, kShadePlainThreads, 0, stream>>>(w, st, b);
-                else wf_shade<kFeatAll><<<g_grid.shade, kShadeThreads, 0, stream>>>(w, st, b);
+                if (nrc) wf_shade_nrc<<<bs, ts, 0, stream>>>(w, st, b, *nrc);
+                else if (feat == 0u) wf_shade<0u><<<bp, tp, 0, stream>>>(w, st, b);
+                else wf_shade<kFeatAll><<<bs, ts, 0, stream>>>(w, st, b);
                 te();
                 if (nrc && !nrc->disabled && (nrc->mode == 1u ? b == 0 : b >= 1)) {  // queries of the paths that stopped here
                     tb(3);
@@ -263,7 +280,7 @@ cudaError_t launch_wavefront(const DevScene& s, const gbrt_ubo& ubo, const Rende
                     if ((e = cudaStreamWaitEvent(side->stream, side->shaded, 0)) != cudaSuccess) return e;
                     ss = side->stream;
                 }
-                GBRT_TRACE_LAUNCH(wf_shadow, g_grid.shadow, ss, w, st, b);
+                GBRT_TRACE_LAUNCH(wf_shadow, gh.blocks, gh.threads, ss, w, st, b);
                 if (side && (e = cudaEventRecord(side->shadowed, ss)) != cudaSuccess) return e;
                 te();
             }

@@ -34,16 +34,18 @@ constexpr int trace_minb(int) { return GBRT_TRACE_MINB; }
 
 // Launches traversal kernel K in the form `mode` (trace_mode, with
 // kTraceOpaque when nothing in the launch can need the alpha test).
-#define GBRT_TRACE_LAUNCH(K, grid, strm, ...)                                                       \
+#define GBRT_TRACE_LAUNCH(K, grid, threads, strm, ...)                                              \
     switch (mode) {                                                                                 \
-        case kTraceWide: K<kTraceWide><<<grid, 128, 0, strm>>>(__VA_ARGS__); break;                 \
-        case kTraceWideTlas: K<kTraceWideTlas><<<grid, 128, 0, strm>>>(__VA_ARGS__); break;         \
-        case kTraceBinary: K<kTraceBinary><<<grid, 128, 0, strm>>>(__VA_ARGS__); break;             \
-        case kTraceWide | kTraceOpaque: K<kTraceWide | kTraceOpaque><<<grid, 128, 0, strm>>>(__VA_ARGS__); break; \
-        case kTraceWideTlas | kTraceOpaque:                                                         \
-            K<kTraceWideTlas | kTraceOpaque><<<grid, 128, 0, strm>>>(__VA_ARGS__);                  \
+        case kTraceWide: K<kTraceWide><<<grid, threads, 0, strm>>>(__VA_ARGS__); break;             \
+        case kTraceWideTlas: K<kTraceWideTlas><<<grid, threads, 0, strm>>>(__VA_ARGS__); break;     \
+        case kTraceBinary: K<kTraceBinary><<<grid, threads, 0, strm>>>(__VA_ARGS__); break;         \
+        case kTraceWide | kTraceOpaque:                                                             \
+            K<kTraceWide | kTraceOpaque><<<grid, threads, 0, strm>>>(__VA_ARGS__);                  \
             break;                                                                                  \
-        default: K<kTraceBinary | kTraceOpaque><<<grid, 128, 0, strm>>>(__VA_ARGS__); break;        \
+        case kTraceWideTlas | kTraceOpaque:                                                         \
+            K<kTraceWideTlas | kTraceOpaque><<<grid, threads, 0, strm>>>(__VA_ARGS__);              \
+            break;                                                                                  \
+        default: K<kTraceBinary | kTraceOpaque><<<grid, threads, 0, strm>>>(__VA_ARGS__); break;    \
     }
 
 // With the ray-sort key, shadow rays are grouped by octant too; shade blocks
@@ -172,9 +174,9 @@ GB_D void flush_trace_stats(const TraceStats& ts, DeviceCounters* c) {
     const unsigned long long tris = warp_sum<unsigned long long>(ts.tris);
     uint32_t stat = ts.status;
     for (int o = 16; o > 0; o >>= 1) stat |= __shfl_down_sync(0xFFFFFFFFu, stat, o);
-    if (lane_id() == 0) {
-        atomicAdd(&c->nodes, nodes);
-        atomicAdd(&c->tris, tris);
+    if (lane_id() == 0) {  // a warp without rays leaves the shared counters alone
+        if (nodes) atomicAdd(&c->nodes, nodes);
+        if (tris) atomicAdd(&c->tris, tris);
         if (stat) atomicOr(&c->status, stat);
     }
 }
@@ -220,19 +222,32 @@ GB_D void initial_state(const gbrt_ubo& ubo, float seed_bits, uint32_t sample, f
     rg = make_uint4(ubo.antialiasing ? 2u : 0u, 0u, tea16(sample, 0x9E3779B9u), 0u);
 }
 
+// Whether a queue of n rays has none left to take, read without the atomic
+// that taking one needs: thousands of warps adding to one word that is past
+// the end anyway took longer than the rays of a small wave.  Uniform in the
+// warp, like the traversal it guards.
+GB_D bool queue_done(const uint32_t* cursor, uint32_t n) {
+    return n == 0u || __shfl_sync(0xFFFFFFFFu, __ldcg(cursor), 0) >= n;
+}
+
 // traceRayEXT for the extension queue of bounce b (closest hit).
 template <int kMode, class Wv>
 GB_D void extend_body(const Wv& w, const WfState& st, uint32_t b, uint32_t jb) {
     const WaveJob& J = w.job(jb);
     uint32_t* cnt = st.counts + jb * kWfCounters;
     const uint32_t n = cnt[kQueue + b], R = J.path0;
+    if (blockIdx.x == w.blk0(0, jb) && threadIdx.x == 0 && n) {
+        if (b == 0) atomicAdd(&J.out.counters->camera, (unsigned long long)n);
+        else atomicAdd(&J.out.counters->extension, (unsigned long long)n);
+    }
+    if (queue_done(&cnt[kWorkExt + b], n)) return;
     const float4* __restrict__ ro = st.ray_o[b & 1] + R;
     const float4* __restrict__ rd = st.ray_d[b & 1] + R;
     TraceStats ts{0, 0, 0};
     // the any-hit context (pixel and sample of a BLEND draw) is only read when an alpha test can run
     const bool alpha = !(J.flags & GBRT_RAY_OPAQUE) && !J.s.all_opaque;
     world_trace<false, kMode>(
-        J.s, n, &cnt[kWorkExt + b], J.flags, ts,
+        J.s, n, &cnt[kWorkExt + b], J.flags, ts, w.nblk(0, jb) * (blockDim.x >> 5),
         [&](uint32_t q, float3& o, float3& d, float& tmin, float& tmax, AnyCtx& ctx) {
             const float4 o4 = ro[q], d4 = rd[q];
             o = f3(o4);
@@ -260,10 +275,6 @@ GB_D void extend_body(const Wv& w, const WfState& st, uint32_t b, uint32_t jb) {
             }
         });
     flush_trace_stats(ts, J.out.counters);
-    if (blockIdx.x == w.blk0(0, jb) && threadIdx.x == 0) {
-        if (b == 0) atomicAdd(&J.out.counters->camera, (unsigned long long)n);
-        else atomicAdd(&J.out.counters->extension, (unsigned long long)n);
-    }
 }
 
 // Closest-hit / miss shading and the rest of rgen's bounce loop
@@ -303,7 +314,7 @@ GB_D void shade_body(const Wv& w, const WfState& st, uint32_t b, const NrcWave* 
     __shared__ uint32_t s_key[2][34];
     uint32_t parity = 0;
     if (sort_rays) {  // block-uniform
-        if (threadIdx.x < 68) (&s_key[0][0])[threadIdx.x] = 0;
+        for (uint32_t i = threadIdx.x; i < 68; i += blockDim.x) (&s_key[0][0])[i] = 0;
         __syncthreads();
     }
     // block-uniform trip count (block_append2_by_key synchronises the block)
@@ -490,13 +501,16 @@ GB_D void shadow_body(const Wv& w, const WfState& st, uint32_t b, uint32_t jb) {
     const WaveJob& J = w.job(jb);
     uint32_t* cnt = st.counts + jb * kWfCounters;
     const uint32_t n = cnt[kShadow + b], R = J.path0;
+    if (blockIdx.x == w.blk0(2, jb) && threadIdx.x == 0 && n)
+        atomicAdd(&J.out.counters->shadow, (unsigned long long)n);
+    if (queue_done(&cnt[kWorkSh + b], n)) return;
     const float4* __restrict__ so = st.sh_o + R;
     const float4* __restrict__ sd = st.sh_d + R;
     TraceStats ts{0, 0, 0};
     const uint32_t flags = GBRT_RAY_TERMINATE_ON_FIRST | J.flags;
     const bool alpha = !(J.flags & GBRT_RAY_OPAQUE) && !J.s.all_opaque;
     world_trace<true, kMode>(
-        J.s, n, &cnt[kWorkSh + b], flags, ts,
+        J.s, n, &cnt[kWorkSh + b], flags, ts, w.nblk(2, jb) * (blockDim.x >> 5),
         [&](uint32_t q, float3& o, float3& d, float& tmin, float& tmax, AnyCtx& ctx) {
             const float4 o4 = so[q], d4 = sd[q];
             o = f3(o4);
@@ -526,8 +540,6 @@ GB_D void shadow_body(const Wv& w, const WfState& st, uint32_t b, uint32_t jb) {
             st.rad[pid] = f4(rad, r.w);
         });
     flush_trace_stats(ts, J.out.counters);
-    if (blockIdx.x == w.blk0(2, jb) && threadIdx.x == 0)
-        atomicAdd(&J.out.counters->shadow, (unsigned long long)n);
 }
 
 // Per pixel of every segment: add its samples' radiance to the job's frame

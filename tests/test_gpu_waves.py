@@ -1,0 +1,46 @@
+"""Waves and ray queries of every size class against the CPU oracle: a single
+ray or path, counts around a warp and around two rays per resident warp
+(152 SMs x 28 warps), where launches change shape, and images whose width and
+height leave remainders in blocks and bands."""
+import numpy as np
+import pytest
+
+import parity
+from rustracer_gb300 import scenes, types as T
+from test_gpu_render import oracle_ref, render_gpu
+from test_gpu_trace import assert_hits_equal, oracle_scene
+
+pytestmark = pytest.mark.gpu
+
+COUNTS = [1, 2, 3, 31, 32, 33, 129, 8511, 8513, 136_197]
+
+
+@pytest.fixture(scope="module")
+def soup():
+    sd = scenes.random_soup(3000, seed=21, size=0.1, alpha_mask_fraction=0.5)
+    rays = scenes.random_rays(max(COUNTS), seed=22)
+    return sd, rays, oracle_scene(sd).trace(rays)[0]
+
+
+@pytest.mark.parametrize("count", COUNTS)
+def test_ray_counts(gpu_ctx, soup, count):
+    from rustracer_gb300 import gbrt
+    sd, rays, ref = soup
+    sc = gbrt.Scene(gpu_ctx, sd)
+    hits, _ = sc.trace(rays[:count])
+    assert_hits_equal(hits, ref[:count])
+    any_hits, _ = sc.trace(rays[:count], 0x4)
+    assert np.array_equal(any_hits["instance_id"] == 0xFFFFFFFF, ref[:count]["instance_id"] == 0xFFFFFFFF)
+
+
+@pytest.mark.parametrize("width,height,spp", [(1, 1, 1), (1, 9, 2), (9, 1, 3), (31, 17, 1), (33, 8, 3), (8, 33, 2),
+                                              (257, 65, 1)])
+def test_frame_sizes(gpu_ctx, width, height, spp):
+    sd = scenes.icosphere_scene(subdiv=2)
+    ubo = sd.ubo(width, height, samples=spp, bounces=6, exposure=1.0)
+    orc, ref = oracle_ref(sd, ubo, width, height)
+    r = render_gpu(gpu_ctx, sd, ubo, width, height)
+    assert_hits_equal(r["hits"].reshape(-1), ref["hits"].reshape(-1))
+    c = parity.classify(r["samples"], ref, orc, ubo, width, height)
+    assert c["unexplained"] == 0, c
+    assert int(r["stats"]["rays_camera"]) == width * height * spp
