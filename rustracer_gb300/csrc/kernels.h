@@ -76,8 +76,10 @@ struct WaveJob {
     float tfar;
     uint32_t path0, npaths;
 };
-// k samples [sample0, sample0 + k) of the pixels [px0, px0 + npw) of a job;
-// path path0 + j * npw + i is sample j of pixel px0 + i.
+// k samples [sample0, sample0 + k) of the pixels at places [px0, px0 + npw) of
+// a job's pixel order (pixel_at); path path0 + i * k + j is sample j of the
+// pixel at place px0 + i: the samples of a pixel are neighbours, and so are
+// the pixels of a tile.
 struct WaveSeg {
     uint32_t path0, job, px0, npw, sample0, si0, k, fin0;  // fin0: first thread of wf_finish
 };

@@ -150,22 +150,39 @@ constexpr int kWorkSh = 96;   // [kWorkSh + b]: fetch cursor of shadow(b)
 constexpr int kMaxBounces = 31;
 constexpr uint32_t kPidMask = kMaxWavePaths - 1u;
 
+// Rows of a band of the pixel order.  Against row-major pixels with the
+// samples outermost, tiles with a pixel's samples together keep the rays of a
+// block (its runs of equal octant, its gathers while shading) close: 1280 x
+// 720 x 16 instanced tori 20.6 -> 18.9 ms, 1080p x 64 icosphere 97.1 -> 93.5,
+// 640 x 360 x 4 cached 3.8 -> 3.1.  Bands of 4 and 16 rows measured the same.
+constexpr uint32_t kBand = 8;
+
+// Pixel at place `i` of a wave's pixel order: bands of kBand rows, column by
+// column, so that consecutive paths cover compact tiles of the image.
+GB_D uint2 pixel_at(uint32_t i, uint32_t W, uint32_t H) {
+    const uint32_t band = i / (kBand * W), r = i - band * (kBand * W), y0 = band * kBand;
+    const uint32_t rows = min(kBand, H - y0);
+    const uint32_t x = rows == kBand ? r / kBand : r / rows;
+    return make_uint2(x, y0 + (r - x * rows));
+}
+
 struct PathXY {
     uint32_t pid, pix, x, y, j;  // wave path, pixel, coordinates, sample within the segment
     const WaveSeg* sg;
 };
 
-// Decodes a queue word (path id | segment << kPidBits) of a job with image width W.
+// Decodes a queue word (path id | segment << kPidBits) of a job with an image of W x H pixels.
 template <class Wv>
-GB_D PathXY decode_path(const Wv& w, uint32_t word, uint32_t W) {
+GB_D PathXY decode_path(const Wv& w, uint32_t word, uint32_t W, uint32_t H) {
     PathXY r;
     r.pid = word & kPidMask;
     r.sg = &w.seg(word >> kPidBits);
-    const uint32_t local = r.pid - r.sg->path0;
-    r.j = local / r.sg->npw;
-    r.pix = r.sg->px0 + (local - r.j * r.sg->npw);
-    r.y = r.pix / W;
-    r.x = r.pix - r.y * W;
+    const uint32_t local = r.pid - r.sg->path0, i = local / r.sg->k;
+    r.j = local - i * r.sg->k;
+    const uint2 xy = pixel_at(r.sg->px0 + i, W, H);
+    r.x = xy.x;
+    r.y = xy.y;
+    r.pix = xy.y * W + xy.x;
     return r;
 }
 
@@ -191,9 +208,8 @@ GB_D void camera_body(const Wv& w, const WfState& st, uint32_t pid) {
     const WaveJob& J = w.job(sg.job);
     if (pid == J.path0) st.counts[sg.job * kWfCounters + kQueue] = J.npaths;
     const uint32_t W = J.out.width;
-    const uint32_t local = pid - sg.path0, j = local / sg.npw, pix = sg.px0 + (local - j * sg.npw);
-    const uint32_t y = pix / W, x = pix - y * W;
-    const uint32_t sample = sg.sample0 + j;
+    const PathXY P = decode_path(w, pid | si << kPidBits, W, J.out.height);
+    const uint32_t x = P.x, y = P.y, sample = sg.sample0 + P.j;
     uint32_t seed = tea16(tea16(x, y), sample);
     uint4 rng = make_uint4(x, y, sample, 0u);
     float3 o, d;
@@ -255,7 +271,7 @@ GB_D void extend_body(const Wv& w, const WfState& st, uint32_t b, uint32_t jb) {
             tmin = 0.001f;
             tmax = J.tfar;
             if (alpha) {
-                const PathXY P = decode_path(w, __float_as_uint(d4.w), J.out.width);
+                const PathXY P = decode_path(w, __float_as_uint(d4.w), J.out.width, J.out.height);
                 ctx = AnyCtx{P.x, P.y, P.sg->sample0 + P.j, b};
             }
         },
@@ -263,7 +279,7 @@ GB_D void extend_body(const Wv& w, const WfState& st, uint32_t b, uint32_t jb) {
             st.hit[R + q] = f4(hit ? h.t : -1.0f, h.u, h.v, __uint_as_float(hit ? h.inst : 0xFFFFFFFFu));
             st.hit_prim[R + q] = h.prim;
             if (b == 0 && J.out.primary_hits) {
-                const PathXY P = decode_path(w, __float_as_uint(rd[q].w), J.out.width);
+                const PathXY P = decode_path(w, __float_as_uint(rd[q].w), J.out.width, J.out.height);
                 gbrt_hit g;
                 g.t = hit ? h.t : -1.0f;
                 g.u = hit ? h.u : 0.0f;
@@ -335,7 +351,7 @@ GB_D void shade_body(const Wv& w, const WfState& st, uint32_t b, const NrcWave* 
             const float4 d4 = rd[q];
             const float3 d = f3(d4);
             word = __float_as_uint(d4.w);
-            const PathXY P = decode_path(w, word, J.out.width);
+            const PathXY P = decode_path(w, word, J.out.width, J.out.height);
             const uint32_t pid = P.pid;
             const float4 h4 = st.hit[R + q];
             float4 tp4, rad4, hp4;
@@ -518,7 +534,7 @@ GB_D void shadow_body(const Wv& w, const WfState& st, uint32_t b, uint32_t jb) {
             tmin = 0.1f;
             tmax = o4.w;
             if (alpha) {
-                const PathXY P = decode_path(w, __float_as_uint(d4.w), J.out.width);
+                const PathXY P = decode_path(w, __float_as_uint(d4.w), J.out.width, J.out.height);
                 ctx = AnyCtx{P.x, P.y, P.sg->sample0 + P.j, b | 0x100u};
             }
         },
@@ -549,12 +565,14 @@ GB_D void finish_body(const Wv& w, const WfState& st, uint32_t i, const NrcWave*
     if (i >= w.nfin()) return;
     const WaveSeg& sg = w.seg(w.seg_of_fin(i));
     const WaveJob& J = w.job(sg.job);
-    const uint32_t li = i - sg.fin0, pix = sg.px0 + li;
+    const uint32_t li = i - sg.fin0;
+    const uint2 xy = pixel_at(sg.px0 + li, J.out.width, J.out.height);
+    const uint32_t pix = xy.y * J.out.width + xy.x;
     float4 acc = J.frame_sum[pix];
     float3 sum = f3(acc);
     float last_t = acc.w;
     for (uint32_t j = 0; j < sg.k; ++j) {
-        const uint32_t pid = sg.path0 + li + j * sg.npw;
+        const uint32_t pid = sg.path0 + li * sg.k + j;
         const float4 r4 = st.rad[pid];
         const float3 r = f3(r4);
         if (J.out.sample_radiance) {
