@@ -19,17 +19,11 @@
 namespace gbrt {
 
 constexpr int kEmpty = 0x7FFFFFFF;  // "stack exhausted"
-// icosphere frame (8-wide, clustered BVH, 7 blocks per SM): 4 / 8 / 12 / 16 /
-// 20 / 24 idle lanes gave 4034 / 4174 / 4225 / 4288 / 4262 / 4183 Mrays/s
-// Entries of the 8-wide traversal stack kept in shared memory (0: the whole
-// stack in local memory, which stays in L1).  Icosphere frame: 4254 Mrays/s
-// with 0, 4258 with 8, 4256 with 16 (noise), so L1 keeps its capacity for
-// nodes and triangles.
-#ifndef GBRT_CW_SMEM_STACK
-#define GBRT_CW_SMEM_STACK 0
-#endif
+// Idle lanes that trigger a refill: icosphere frame at 12 / 16 / 20 lanes 86.1 /
+// 86.5 / 88.1 ms, instanced tori 13.6 / 13.7 / 14.0 ms (with triangles tested
+// lane by lane 16 was best: the idle lanes now work).
 #ifndef GBRT_REFILL
-#define GBRT_REFILL 16
+#define GBRT_REFILL 12
 #endif
 constexpr uint32_t kRefill = GBRT_REFILL;  // idle lanes that trigger a refill
 
@@ -218,35 +212,50 @@ GB_D void persistent_trace(const DevScene& s, uint32_t n, uint32_t* work, uint32
 
 namespace gbrt {
 
+// Inclusive prefix sum over the warp.
+GB_D uint32_t warp_scan(uint32_t v) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+        asm volatile("{\n.reg .u32 t;\n.reg .pred p;\nshfl.sync.up.b32 t|p, %0, %1, 0, 0xFFFFFFFF;\n@p add.u32 %0, %0, t;\n}\n"
+                     : "+r"(v)
+                     : "r"(o));
+    return v;
+}
+
+// What the lanes of a warp need of each other's rays to test triangles for
+// one another, and the triangles of one round.
+struct WarpTris {
+    float4 o[32];     // origin, tmin
+    float4 s[32];     // shear constants, axis permutation kx | ky << 2 | kz << 4
+    uint2 pair[32];   // triangle slot, lane of its ray
+};
+
 // Persistent-lane traversal of the 8-wide world BVH; same interface and
 // refill policy as persistent_trace.
-template <bool kAny, bool kTlas, bool kAlpha, class Loader, class Finisher>
+//
+// Every lane visits the nodes of its own ray, but the triangles that a step
+// of the warp turned up (none to a dozen a lane) are dealt out over all 32
+// lanes through shared memory, one each: the kernel is bound by instruction
+// issue, and testing them lane by lane kept about 4 of 32 lanes busy while the
+// lane with the most triangles finished.  The owner of a ray then takes the
+// results of its triangles in slot order, so hits are those of the
+// lane-by-lane loop.  Icosphere frame (1080p x 64): extend 41.5 -> 36.7 ms,
+// shadow 22.4 -> 18.0; 1.5M incoherent ray queries 383 -> 310 us.  kHit: the finisher reads the hit
+// of an any-hit query, not only whether there is one.  Every block has at
+// most 128 threads.
+template <bool kAny, bool kTlas, bool kAlpha, bool kHit, class Loader, class Finisher>
 GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uint32_t flags, TraceStats& ts,
                               uint32_t quota, Loader&& load, Finisher&& finish) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu, kInner = 0xFF000000u;
+    __shared__ WarpTris s_tris[4];
+    WarpTris& sw = s_tris[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
     const bool test_alpha = kAlpha && !(flags & GBRT_RAY_OPAQUE) && !s.all_opaque;
-#if GBRT_CW_SMEM_STACK
-    // the top kSmemStack entries of each lane's stack in shared memory ([entry][thread]: a warp's accesses
-    // to one depth are consecutive 8-byte words), deeper ones in local memory; every traversal kernel
-    // runs 128-thread blocks (its launch bound)
-    constexpr int kSmemStack = GBRT_CW_SMEM_STACK;
-    __shared__ uint2 s_stack[kSmemStack][128];
-    uint2 stack[kCwStack - kSmemStack];
-    auto push = [&](uint2 v, int i) {
-        if (i < kSmemStack) s_stack[i][threadIdx.x] = v;
-        else stack[i - kSmemStack] = v;
-    };
-    auto pop = [&](int i) { return i < kSmemStack ? s_stack[i][threadIdx.x] : stack[i - kSmemStack]; };
-#else
     uint2 stack[kCwStack];
-    auto push = [&](uint2 v, int i) { stack[i] = v; };
-    auto pop = [&](int i) { return stack[i]; };
-#endif
     bool has = false, exhausted = false;
     uint32_t q = 0, oct = 0;
     TRay r;
     Hit best;
-    float best_det = 1.0f;  // any-hit queries: best.u, best.v hold V, W of the world hit until the ray is done
     AnyCtx ctx{0, 0, 0, 0};
     float tmin = 0.0f, tmax = 0.0f;
     uint2 ng = make_uint2(0, 0);
@@ -254,12 +263,12 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
     uint32_t iter = 0;
     for (;;) {
         if (!exhausted) {
-            const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !has);
+            const uint32_t idle = __ballot_sync(kAll, !has);
             if (__popc(idle) >= (int)kRefill) {
                 const uint32_t take = min((uint32_t)__popc(idle), quota);
                 uint32_t base = 0;
                 if (lane == 0) base = atomicAdd(work, take);
-                base = __shfl_sync(0xFFFFFFFFu, base, 0);
+                base = __shfl_sync(kAll, base, 0);
                 if (base + take >= n) exhausted = true;
                 const uint32_t rank = __popc(idle & ((1u << lane) - 1u));
                 if (!has && rank < take) {
@@ -269,7 +278,6 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
                         load(q, o, d, tmin, tmax, ctx);
                         best.t = tmax;
                         best.u = best.v = 0.0f;
-                        best_det = 1.0f;
                         best.inst = best.prim = best.bgeo = 0xFFFFFFFFu;
                         iter = 0;
                         if (d.x == 0.0f && d.y == 0.0f && d.z == 0.0f) {
@@ -278,6 +286,8 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
                             has = true;
                             setup_ray(r, o, d);
                             oct = (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
+                            sw.o[lane] = make_float4(o.x, o.y, o.z, tmin);
+                            sw.s[lane] = make_float4(r.Sx, r.Sy, r.Sz, __int_as_float(r.kx | r.ky << 2 | r.kz << 4));
                             sp = 0;
                             // virtual parent: one inner child (the root, node 0) in slot 0
                             ng = s.has_world ? make_uint2(0u, (1u << (24u + oct)) | 1u) : make_uint2(0u, 0u);
@@ -286,72 +296,123 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
                 }
             }
         }
-        if (!__any_sync(0xFFFFFFFFu, has)) {
+        if (!__any_sync(kAll, has)) {
             if (exhausted) break;
             continue;
         }
-        if (!has) continue;
+        // --- one node per ray -------------------------------------------------
         bool done = false;
-        while (!(ng.y & 0xFF000000u) && sp > 0) ng = pop(--sp);
-        if (!(ng.y & 0xFF000000u)) {
-            done = true;
-        } else if (++iter > kMaxIter) {
-            ts.status |= GBRT_STATUS_ITER_LIMIT;
-            done = true;
-        } else {
-            const uint32_t bit = __ffs(ng.y & 0xFF000000u) - 1u;
-            ng.y &= ~(1u << bit);
-            const uint32_t slot = (bit - 24u) ^ oct;
-            const uint32_t child = ng.x + __popc((ng.y & 0xFFu) & ((1u << slot) - 1u));
-            if (ng.y & 0xFF000000u) {
-                if (sp < kCwStack) push(ng, sp++);
-                else ts.status |= GBRT_STATUS_STACK_OVERFLOW;
+        uint32_t tri_bits = 0, tri_base = 0;
+        if (has) {
+            if (!(ng.y & kInner) && sp > 0) ng = stack[--sp];
+            if (++iter > kMaxIter) {
+                ts.status |= GBRT_STATUS_ITER_LIMIT;
+                done = true;
+            } else if (ng.y & kInner) {
+                const uint32_t bit = __ffs(ng.y & kInner) - 1u;
+                ng.y &= ~(1u << bit);
+                const uint32_t slot = (bit - 24u) ^ oct;
+                const uint32_t child = ng.x + __popc((ng.y & 0xFFu) & ((1u << slot) - 1u));
+                if (ng.y & kInner) {
+                    if (sp < kCwStack) stack[sp++] = ng;
+                    else ts.status |= GBRT_STATUS_STACK_OVERFLOW;
+                }
+                uint32_t cb, im;
+                const uint32_t hm = cw_intersect(s.cw_nodes, child, r, oct, tmin, best.t, cb, tri_base, im);
+                ts.nodes++;
+                ng = make_uint2(cb, (hm & kInner) | im);
+                tri_bits = hm & 0x00FFFFFFu;
             }
-            uint32_t cb, tb, im;
-            const uint32_t hm = cw_intersect(s.cw_nodes, child, r, oct, tmin, best.t, cb, tb, im);
-            ts.nodes++;
-            ng = make_uint2(cb, (hm & 0xFF000000u) | im);
-            uint32_t tri_bits = hm & 0x00FFFFFFu;
-            while (tri_bits) {
+        }
+        // --- the triangles of all rays, 32 at a time ----------------------------
+        const uint32_t cnt = __popc(tri_bits);
+        const uint32_t incl = warp_scan(cnt), total = __shfl_sync(kAll, incl, 31);
+        uint32_t pos = incl - cnt;  // place of this lane's next triangle in the round
+        for (uint32_t base = 0; base < total; base += 32) {
+            uint32_t mine = 0;
+            while (tri_bits && pos < 32u) {
                 const uint32_t tbit = __ffs(tri_bits) - 1u;
                 tri_bits &= tri_bits - 1u;
-                const TriRec* tr = s.cw_tris + tb + tbit;
-                const float4 pa = __ldg(&tr->a), pb = __ldg(&tr->b), pc = __ldg(&tr->c);
+                sw.pair[pos] = make_uint2(tri_base + tbit, lane);
+                mine |= 1u << pos;
+                ++pos;
+            }
+            pos -= 32u;
+            __syncwarp();
+            const bool live = lane < total - base;
+            uint2 pr = make_uint2(0u, lane);
+            if (live) pr = sw.pair[lane];
+            const float tcur = __shfl_sync(kAll, best.t, pr.y);
+            AnyCtx pc{0, 0, 0, 0};
+            if (kAlpha && test_alpha)
+                pc = AnyCtx{__shfl_sync(kAll, ctx.px, pr.y), __shfl_sync(kAll, ctx.py, pr.y),
+                            __shfl_sync(kAll, ctx.sample, pr.y), __shfl_sync(kAll, ctx.tag, pr.y)};
+            bool hit = false;
+            float t = 0.0f, u = 0.0f, v = 0.0f;
+            uint32_t inst = 0, prim = 0;
+            if (live) {
+                const float4 po = sw.o[pr.y], ps = sw.s[pr.y];
+                const int k = __float_as_int(ps.w);
+                TRay pray;
+                pray.o = f3(po);
+                pray.Sx = ps.x;
+                pray.Sy = ps.y;
+                pray.Sz = ps.z;
+                pray.kx = k & 3;
+                pray.ky = (k >> 2) & 3;
+                pray.kz = k >> 4;
+                const TriRec* tr = s.cw_tris + pr.x;
+                const float4 pa = __ldg(&tr->a), pb = __ldg(&tr->b), pcv = __ldg(&tr->c);
                 ts.tris++;
-                // any-hit queries keep V, W and det of the hit and divide once the ray is done (if
-                // their caller reads u, v at all); closest-hit queries divide per accepted hit
-                float t, u, v, det = 1.0f;
-                if constexpr (kAny) {
-                    if (!isect_tri_t(r, f3(pa), f3(pb), f3(pc), tmin, best.t, t, u, v, det)) continue;
+                inst = __float_as_uint(pa.w);
+                prim = __float_as_uint(pb.w);
+                if constexpr (kAny && !kHit && !kAlpha) {
+                    float V, W, det;
+                    hit = isect_tri_t(pray, f3(pa), f3(pb), f3(pcv), po.w, tcur, t, V, W, det);
                 } else {
-                    if (!isect_tri(r, f3(pa), f3(pb), f3(pc), tmin, best.t, t, u, v)) continue;
+                    hit = isect_tri(pray, f3(pa), f3(pb), f3(pcv), po.w, tcur, t, u, v);
+                    if (kAlpha && hit && test_alpha && !(__float_as_uint(pcv.w) >> 31) &&
+                        anyhit_ignore(s, s.inst[inst].custom, prim, inst, u, v, pc))
+                        hit = false;
                 }
-                const uint32_t inst = __float_as_uint(pa.w);
-                const uint32_t prim = __float_as_uint(pb.w);
-                const uint32_t gw = __float_as_uint(pc.w);
-                if (!closer(t, inst, prim, best)) continue;
-                if (test_alpha && !(gw >> 31) &&
-                    anyhit_ignore(s, s.inst[inst].custom, prim, inst, kAny ? __fdiv_rn(u, det) : u,
-                                  kAny ? __fdiv_rn(v, det) : v, ctx))
-                    continue;
-                best.t = t;
-                best.u = u;
-                best.v = v;
-                best_det = det;
-                best.inst = inst;
-                best.prim = prim;
-                best.bgeo = gw & 0x7FFFFFFFu;
-                if (kAny) {
-                    done = true;
-                    break;
+            }
+            uint32_t my = __ballot_sync(kAll, hit) & mine;  // hits of this lane's own ray
+            __syncwarp();                                   // the pairs have been read
+            if constexpr (kAny) {
+                if constexpr (kHit) {
+                    const uint32_t f = my && !done ? __ffs(my) - 1u : lane;
+                    const float t2 = __shfl_sync(kAll, t, f), u2 = __shfl_sync(kAll, u, f),
+                                v2 = __shfl_sync(kAll, v, f);
+                    const uint32_t i2 = __shfl_sync(kAll, inst, f), p2 = __shfl_sync(kAll, prim, f);
+                    if (my && !done) {
+                        best.t = t2;
+                        best.u = u2;
+                        best.v = v2;
+                        best.inst = i2;
+                        best.prim = p2;
+                    }
+                } else if (my) {
+                    best.inst = 0u;
+                }
+                done = done || my;
+            } else {
+                while (__any_sync(kAll, my != 0u)) {
+                    const uint32_t f = my ? __ffs(my) - 1u : lane;
+                    const float t2 = __shfl_sync(kAll, t, f), u2 = __shfl_sync(kAll, u, f),
+                                v2 = __shfl_sync(kAll, v, f);
+                    const uint32_t i2 = __shfl_sync(kAll, inst, f), p2 = __shfl_sync(kAll, prim, f);
+                    if (my && closer(t2, i2, p2, best)) {
+                        best.t = t2;
+                        best.u = u2;
+                        best.v = v2;
+                        best.inst = i2;
+                        best.prim = p2;
+                    }
+                    my &= my - 1u;
                 }
             }
         }
-        if (done) {
-            if constexpr (kAny) {
-                best.u = __fdiv_rn(best.u, best_det);
-                best.v = __fdiv_rn(best.v, best_det);
-            }
+        if (has && (done || (!(ng.y & kInner) && sp == 0))) {
             if constexpr (kTlas) {
                 if (s.has_tlas && !(kAny && best.inst != 0xFFFFFFFFu))
                     trace_tlas<kAny, true>(s, r, r.o, r.d, tmin, best, test_alpha, ctx, ts);
@@ -372,14 +433,14 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
 // code it leaves out cost the 8-wide traversal kernels spills.
 constexpr int kTraceBinary = 0, kTraceWide = 1, kTraceWideTlas = 2, kTraceOpaque = 4;
 
-template <bool kAny, int kMode, class Loader, class Finisher>
+template <bool kAny, int kMode, bool kHit, class Loader, class Finisher>
 GB_D void world_trace(const DevScene& s, uint32_t n, uint32_t* work, uint32_t flags, TraceStats& ts,
                       uint32_t warps, Loader&& load, Finisher&& finish) {
     constexpr int kForm = kMode & 3;
     constexpr bool kAlpha = !(kMode & kTraceOpaque);
     const uint32_t quota = ray_quota(n, warps);
     if constexpr (kForm == kTraceBinary) persistent_trace<kAny, kAlpha>(s, n, work, flags, ts, quota, load, finish);
-    else persistent_trace_cw<kAny, kForm == kTraceWideTlas, kAlpha>(s, n, work, flags, ts, quota, load, finish);
+    else persistent_trace_cw<kAny, kForm == kTraceWideTlas, kAlpha, kHit>(s, n, work, flags, ts, quota, load, finish);
 }
 
 // Launch shape of a traversal kernel over at most n rays, `resident` blocks

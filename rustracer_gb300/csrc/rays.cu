@@ -11,7 +11,7 @@ __global__ void __launch_bounds__(128) trace_rays_persistent(DevScene s, const g
                                                              uint32_t flags, gbrt_hit* hits, uint32_t* work,
                                                              DeviceCounters* cnt) {
     TraceStats ts{0, 0, 0};
-    world_trace<kAny, kMode>(
+    world_trace<kAny, kMode, true>(
         s, n, work, flags, ts, gridDim.x * (blockDim.x >> 5),
         [&](uint32_t q, float3& o, float3& d, float& tmin, float& tmax, AnyCtx& ctx) {
             const gbrt_ray r = rays[q];

@@ -247,13 +247,14 @@ GB_D uint32_t cw_intersect(const CwNode* nodes, uint32_t node, const TRay& r, ui
     tri_base = w1.y;
     imask = w0.w >> 24;
     // per axis: t = o + q * s = fma(1 + q 2^-15, 2^15 s, o - 2^15 s).  An axis the
-    // ray is parallel to (d = 0) gives (-inf, +inf) and the origin must lie
+    // ray is parallel to (d = 0, which setup_ray turns into inv = +-FLT_MAX; a d
+    // whose inverse rounds to that moves less than a box's padding) gives (-inf, +inf) and the origin must lie
     // inside that child's slab instead.
     const float scx = __uint_as_float((w0.w & 0xFFu) << 23);
     const float scy = __uint_as_float(((w0.w >> 8) & 0xFFu) << 23);
     const float scz = __uint_as_float(((w0.w >> 16) & 0xFFu) << 23);
     const float px = __uint_as_float(w0.x), py = __uint_as_float(w0.y), pz = __uint_as_float(w0.z);
-    const bool zx = r.d.x == 0.0f, zy = r.d.y == 0.0f, zz = r.d.z == 0.0f;
+    const bool zx = fabsf(r.inv.x) == FLT_MAX, zy = fabsf(r.inv.y) == FLT_MAX, zz = fabsf(r.inv.z) == FLT_MAX;
     const float Sx = zx ? 0.0f : 32768.0f * (scx * r.inv.x);
     const float Sy = zy ? 0.0f : 32768.0f * (scy * r.inv.y);
     const float Sz = zz ? 0.0f : 32768.0f * (scz * r.inv.z);

@@ -262,7 +262,7 @@ GB_D void extend_body(const Wv& w, const WfState& st, uint32_t b, uint32_t jb) {
     TraceStats ts{0, 0, 0};
     // the any-hit context (pixel and sample of a BLEND draw) is only read when an alpha test can run
     const bool alpha = !(J.flags & GBRT_RAY_OPAQUE) && !J.s.all_opaque;
-    world_trace<false, kMode>(
+    world_trace<false, kMode, true>(
         J.s, n, &cnt[kWorkExt + b], J.flags, ts, w.nblk(0, jb) * (blockDim.x >> 5),
         [&](uint32_t q, float3& o, float3& d, float& tmin, float& tmax, AnyCtx& ctx) {
             const float4 o4 = ro[q], d4 = rd[q];
@@ -525,7 +525,7 @@ GB_D void shadow_body(const Wv& w, const WfState& st, uint32_t b, uint32_t jb) {
     TraceStats ts{0, 0, 0};
     const uint32_t flags = GBRT_RAY_TERMINATE_ON_FIRST | J.flags;
     const bool alpha = !(J.flags & GBRT_RAY_OPAQUE) && !J.s.all_opaque;
-    world_trace<true, kMode>(
+    world_trace<true, kMode, false>(
         J.s, n, &cnt[kWorkSh + b], flags, ts, w.nblk(2, jb) * (blockDim.x >> 5),
         [&](uint32_t q, float3& o, float3& d, float& tmin, float& tmax, AnyCtx& ctx) {
             const float4 o4 = so[q], d4 = sd[q];

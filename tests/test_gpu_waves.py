@@ -44,3 +44,16 @@ def test_frame_sizes(gpu_ctx, width, height, spp):
     c = parity.classify(r["samples"], ref, orc, ubo, width, height)
     assert c["unexplained"] == 0, c
     assert int(r["stats"]["rays_camera"]) == width * height * spp
+
+
+@pytest.mark.parametrize("ntri,size,masked", [(60, 2.0, 0.0), (600, 0.8, 0.5)])
+def test_crowded_leaves(gpu_ctx, ntri, size, masked):
+    """Big overlapping triangles: a step of a warp turns up far more of them than it has lanes."""
+    from rustracer_gb300 import gbrt
+    sd = scenes.random_soup(ntri, seed=31, size=size, alpha_mask_fraction=masked)
+    rays = scenes.random_rays(20_001, seed=32)
+    ref = oracle_scene(sd).trace(rays)[0]
+    sc = gbrt.Scene(gpu_ctx, sd)
+    assert_hits_equal(sc.trace(rays)[0], ref)
+    any_hits = sc.trace(rays, 0x4)[0]
+    assert np.array_equal(any_hits["instance_id"] == 0xFFFFFFFF, ref["instance_id"] == 0xFFFFFFFF)
