@@ -22,12 +22,13 @@
 #include "persistent.cuh"
 
 // Resident 128-thread blocks per SM the traversal kernels (extend, shadow)
-// are compiled for: 7 gives them 72 registers (a few dozen bytes of spills)
-// at 28 warps per SM.  The traversal waits on dependent node loads, so warps
-// pay more than registers: on the icosphere frame with the clustered BVH,
-// 4 / 5 / 6 / 7 / 8 blocks gave 3472 / 3768 / 4046 / 4159 / 4134 Mrays/s.
+// are compiled for: 8 gives them 64 registers, which the 8-wide forms need (no
+// spills without alpha tests, 20 B with them), at 32 warps per SM to cover
+// dependent node and triangle loads.  6 / 7 / 8 / 9 / 10 blocks: icosphere
+// frame (1080p x 64) 89.9 / 80.3 / 77.3 / 78.8 / 79.7 ms (6 on an earlier form),
+// instanced tori - / 11.6 / 11.4 / 12.3 / 13.5 ms.
 #ifndef GBRT_TRACE_MINB
-#define GBRT_TRACE_MINB 7
+#define GBRT_TRACE_MINB 8
 #endif
 // Same bound for every traversal form.
 constexpr int trace_minb(int) { return GBRT_TRACE_MINB; }
