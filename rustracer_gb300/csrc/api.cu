@@ -182,6 +182,10 @@ void refresh_view(gbrt_scene* s) {
     v.blas_cw_tris = s->blas_cw_nodes.p ? s->blas_cw_tris.as<TriRec>() : nullptr;
 }
 
+// Build scratch that a context keeps between builds: scenes of up to four
+// million triangles rebuild without allocating, larger ones give theirs back.
+constexpr size_t kArenaKeep = size_t(1) << 30;
+
 // Builds the merged world BVH, the BLASes of transformed instances and the
 // TLAS into fresh pools.
 int build_all(gbrt_scene* s) {
@@ -265,23 +269,19 @@ int build_all(gbrt_scene* s) {
     if (!world_items.empty()) {
         CU(c, upload(s->items, world_items.data(), world_items.size(), st), "upload(items)");
         BvhResult r;
-        CU(c, build_triangle_bvh(s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
-                                 s->prims.as<gbrt_priminfo>(), s->items.as<uint4>(), (uint32_t)world_items.size(),
-                                 s->nodes.as<BNode2>(), 0, s->tris.as<TriRec>(), 0, &r, st,
-                                 s->inst.as<DevInstance>()),
+        const size_t nw = world_items.size();
+        CU(c, s->cw_nodes.alloc(nw * sizeof(CwNode)), "cudaMalloc(wide nodes)");
+        CU(c, s->cw_tris.alloc(nw * sizeof(TriRec)), "cudaMalloc(wide triangles)");
+        const WideBuild wide{s->cw_nodes.as<CwNode>(), s->cw_tris.as<TriRec>(), &s->cw_count, &s->cw_levels, cw_width(s)};
+        CU(c, build_triangle_bvh(c->build, s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
+                                 s->prims.as<gbrt_priminfo>(), s->items.as<uint4>(), (uint32_t)nw,
+                                 s->nodes.as<BNode2>(), 0, s->tris.as<TriRec>(), 0, &r, st, s->inst.as<DevInstance>(),
+                                 kBvhPloc, &wide),
            "build world BVH");
         v.has_world = 1;
         v.world_root = r.root;
         v.world_lo = r.lo;
         v.world_hi = r.hi;
-        const size_t nw = world_items.size();
-        CU(c, s->cw_nodes.alloc(nw * sizeof(CwNode)), "cudaMalloc(wide nodes)");
-        CU(c, s->cw_tris.alloc(nw * sizeof(TriRec)), "cudaMalloc(wide triangles)");
-        CU(c, build_triangle_cwbvh(s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
-                                   s->prims.as<gbrt_priminfo>(), s->items.as<uint4>(), (uint32_t)nw,
-                                   s->cw_nodes.as<CwNode>(), s->cw_tris.as<TriRec>(), &s->cw_count, st,
-                                   &s->cw_levels, s->inst.as<DevInstance>(), cw_width(s)),
-           "build wide world BVH");
         s->nworld = (uint32_t)nw;
         // the tree's SAH cost proxy as built (a refit of unchanged vertices rewrites the same nodes), the
         // reference for the drift check of later refits
@@ -325,20 +325,17 @@ int build_all(gbrt_scene* s) {
             for (uint32_t p = 0; p < ntri; ++p) items[p] = make_uint4(0u, g, p, s->ranges[g].opaque ? 1u : 0u);
             CU(c, upload(bitems, items.data(), items.size(), st), "upload(blas items)");
             BvhResult r;
-            CU(c, build_triangle_bvh(s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
+            uint32_t used = 0;
+            const WideBuild wide{s->blas_cw_nodes.as<CwNode>() + cw_node0[g], s->blas_cw_tris.as<TriRec>() + cw_tri0[g],
+                                 &used, nullptr, cw_width(s)};
+            CU(c, build_triangle_bvh(c->build, s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
                                      s->prims.as<gbrt_priminfo>(), bitems.as<uint4>(), ntri, s->nodes.as<BNode2>(),
-                                     blas_node_base[g], s->tris.as<TriRec>(), blas_tri_base[g], &r, st),
+                                     blas_node_base[g], s->tris.as<TriRec>(), blas_tri_base[g], &r, st, nullptr,
+                                     kBvhPloc, &wide),
                "build BLAS");
             broot[g] = r.root;
             blo[g] = r.lo;
             bhi[g] = r.hi;
-            uint32_t used = 0;
-            CU(c, build_triangle_cwbvh(s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
-                                       s->prims.as<gbrt_priminfo>(), bitems.as<uint4>(), ntri,
-                                       s->blas_cw_nodes.as<CwNode>() + cw_node0[g],
-                                       s->blas_cw_tris.as<TriRec>() + cw_tri0[g], &used, st, nullptr, nullptr,
-                                       cw_width(s)),
-               "build wide BLAS");
         }
         const uint32_t nt = (uint32_t)tlas_ids.size();
         std::vector<float4> ilo(nt), ihi(nt);
@@ -363,7 +360,7 @@ int build_all(gbrt_scene* s) {
                                    d_bhi.as<float4>(), nt, d_lo.as<float4>(), d_hi.as<float4>(), st),
            "instance boxes");
         BvhResult r;
-        CU(c, build_instance_bvh(d_lo.as<float4>(), d_hi.as<float4>(), d_ids.as<uint32_t>(), nt,
+        CU(c, build_instance_bvh(c->build, d_lo.as<float4>(), d_hi.as<float4>(), d_ids.as<uint32_t>(), nt,
                                  s->nodes.as<BNode2>(), tlas_node_base, s->tris.as<TriRec>(), tlas_tri_base, &r, st),
            "build TLAS");
         s->tlas_node_base = tlas_node_base;
@@ -378,6 +375,7 @@ int build_all(gbrt_scene* s) {
         s->blas_cw_tris.release();
         CU(c, cudaStreamSynchronize(st), "sync after build");
     }
+    if (c->build.bytes > kArenaKeep) c->build.release();  // the stream has been waited for
     s->h_inst = std::move(hinst);
     s->tlas_ids = std::move(tlas_ids);
     s->flattened = false;
@@ -425,7 +423,7 @@ int update_instances(gbrt_scene* s, const gbrt_instance* in, uint32_t n) {
                                    s->tlas_bhi.as<float4>(), nt, s->tlas_lo.as<float4>(), s->tlas_hi.as<float4>(), st),
            "instance boxes");
         BvhResult r;
-        CU(c, build_instance_bvh(s->tlas_lo.as<float4>(), s->tlas_hi.as<float4>(), s->tlas_ids_d.as<uint32_t>(), nt,
+        CU(c, build_instance_bvh(c->build, s->tlas_lo.as<float4>(), s->tlas_hi.as<float4>(), s->tlas_ids_d.as<uint32_t>(), nt,
                                  s->nodes.as<BNode2>(), s->tlas_node_base, s->tris.as<TriRec>(), s->tlas_tri_base, &r,
                                  st),
            "rebuild TLAS");
@@ -483,8 +481,8 @@ int refit_world(gbrt_scene* s) {
     // binary world BVH: rebuilt (an LBVH over the same items, one launch chain);
     // 8-wide world BVH: refit in place, keeping its topology and slots
     BvhResult r;
-    CU(c, build_triangle_bvh(s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(), s->prims.as<gbrt_priminfo>(),
-                             s->items.as<uint4>(), s->nworld, s->nodes.as<BNode2>(), 0, s->tris.as<TriRec>(), 0, &r,
+    CU(c, build_triangle_bvh(c->build, s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
+                             s->prims.as<gbrt_priminfo>(), s->items.as<uint4>(), s->nworld, s->nodes.as<BNode2>(), 0, s->tris.as<TriRec>(), 0, &r,
                              st, s->inst.as<DevInstance>(), kBvhFast),
        "rebuild world BVH");
     CU(c, s->cw_boxes.reserve((size_t)s->cw_count * 2 * sizeof(float4) + 16), "cudaMalloc(refit boxes)");
@@ -570,6 +568,7 @@ int gbrt_ctx_destroy(gbrt_ctx* c) {
         c->scratch_img.release();
         c->scratch_samples.release();
         c->scratch_phits.release();
+        c->build.release();
         c->wf_mem.release();
         c->wf_frame.release();
         stage_timer_free(c->timer);

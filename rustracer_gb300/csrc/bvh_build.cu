@@ -11,7 +11,7 @@
 // written in the traversal layout (BNode2 with both child boxes; leaves as
 // codes over a contiguous range of TriRec slots in Morton order).
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_scan.cuh>
+#include <cmath>
 #include <cstring>
 #include <utility>
 #include <float.h>
@@ -63,8 +63,20 @@ struct Scratch {
     uint32_t* collapse;   // [n-1] 1 = becomes a leaf
     uint32_t* arrive;     // [n-1]
     uint32_t* cbounds;    // 6 order-encoded centroid bounds
+    TriRec* unsorted;     // [n]
     void* cub_tmp;
     size_t cub_bytes;
+    // 8-wide collapse
+    float* dp_cost;         // [n-1][8]
+    uint8_t* dp_split;      // [n-1][8]
+    uint32_t* cw_collapse;  // [n-1] 1 = one leaf slot of a wide node
+    uint2 *task_a, *task_b; // [n]
+    uint32_t* counters;     // 4
+    // clustering (ploc_build.inc); the boxes share memory with what is written after it
+    int32_t* p_cid[2];
+    float4 *p_lo[2], *p_hi[2];
+    int32_t *p_partner, *p_left, *p_right, *p_parent, *p_lparent;
+    uint32_t *p_cnt, *p_pre, *p_off, *p_loff, *p_tile, *p_state;
 };
 
 // Item i's triangle (world space when `inst` is given and the item's
@@ -205,13 +217,36 @@ __device__ __forceinline__ float half_area(float3 l, float3 h) {
     return e.x * e.y + e.y * e.z + e.z * e.x;
 }
 
+// Wide collapse: costs of a wide node and of a triangle in a leaf slot, per
+// unit of area, and the most triangles a slot holds (cwbvh_build.inc).
+constexpr uint32_t kCwMaxLeaf = 3;
+#ifndef GBRT_CW_COST_NODE
+#define GBRT_CW_COST_NODE 1.0f
+#endif
+#ifndef GBRT_CW_COST_TRI
+#define GBRT_CW_COST_TRI 0.3f
+#endif
+constexpr float kCwCostNode = GBRT_CW_COST_NODE, kCwCostTri = GBRT_CW_COST_TRI;
+
 // Bottom-up: one thread per leaf climbs while it is the second child to
-// arrive at a node.  Child data is read with L1-bypassing loads.
+// arrive at a node.  Child data is read with L1-bypassing loads.  Per inner
+// node: its box, its SAH cost and whether it becomes a leaf of the binary
+// tree; with kWide also the optimal distribution of the wide collapse
+// (cwbvh_build.inc), in the same climb: a climb is bound by its chain of
+// atomics and loads over the tree's depth, so a second one would cost as much
+// again.
+//
+// The distribution: dp_cost[p][j-1] = least cost of p's subtree with at most
+// j slots; dp_split[p][j-1] = 0 when that is the cost with j - 1 slots, else
+// the slots k of the left child (the right one gets j - k); dp_split[p][0] =
+// the left child's slots when p is a wide node (a distribution over `width`
+// slots).  cw_collapse[p] = 1 when p is best a single leaf slot.
+template <bool kWide>
 __global__ void bottom_up_kernel(int n, const uint32_t* idx, const float4* lo, const float4* hi,
                                  const int32_t* left, const int32_t* right, const int32_t* parent_i,
                                  const int32_t* parent_l, const uint32_t* rlo, const uint32_t* rhi, float4* ilo,
-                                 float4* ihi, float* cost, uint32_t* collapse, uint32_t* arrive, uint32_t max_leaf,
-                                 float cost_traverse) {
+                                 float4* ihi, float* cost, uint32_t* collapse, uint32_t* arrive, float* dp_cost,
+                                 uint8_t* dp_split, uint32_t* cw_collapse, int width) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     int p = parent_l[i];
@@ -221,6 +256,7 @@ __global__ void bottom_up_kernel(int n, const uint32_t* idx, const float4* lo, c
         __threadfence();
         float3 bl[2], bh[2];
         float c[2];
+        float4 d[2][2];  // the children's costs with 1..8 slots
         const int32_t ch[2] = {__ldcg(&left[p]), __ldcg(&right[p])};
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
@@ -228,23 +264,80 @@ __global__ void bottom_up_kernel(int n, const uint32_t* idx, const float4* lo, c
                 const uint32_t item = __ldcg(&idx[~ch[k]]);
                 bl[k] = f3(__ldcg(&lo[item]));
                 bh[k] = f3(__ldcg(&hi[item]));
-                c[k] = kCostTri * half_area(bl[k], bh[k]);
+                const float a = half_area(bl[k], bh[k]);
+                c[k] = kCostTri * a;
+                const float w = kCwCostTri * a;  // one triangle: a leaf slot whatever the budget
+                d[k][0] = d[k][1] = f4(w, w, w, w);
             } else {
                 bl[k] = f3(__ldcg(&ilo[ch[k]]));
                 bh[k] = f3(__ldcg(&ihi[ch[k]]));
                 c[k] = __ldcg(&cost[ch[k]]);
+                if constexpr (kWide) {
+                    const float4* q = reinterpret_cast<const float4*>(dp_cost + (size_t)ch[k] * 8);
+                    d[k][0] = __ldcg(q);
+                    d[k][1] = __ldcg(q + 1);
+                }
             }
         }
         const float3 l = fmin3(bl[0], bl[1]), h = fmax3(bh[0], bh[1]);
         const float a = half_area(l, h);
         const uint32_t count = rhi[p] - rlo[p] + 1u;
-        const float split = cost_traverse * a + c[0] + c[1];
+        const float split = kCostTraverse * a + c[0] + c[1];
         const float as_leaf = kCostTri * a * (float)count;
-        const bool col = count <= max_leaf && as_leaf <= split;
+        const bool col = count <= kMaxLeaf && as_leaf <= split;
         ilo[p] = f4(l, 0.0f);
         ihi[p] = f4(h, 0.0f);
         cost[p] = col ? as_leaf : split;
         collapse[p] = col ? 1u : 0u;
+        if constexpr (kWide) {
+            const float cc[2][8] = {{d[0][0].x, d[0][0].y, d[0][0].z, d[0][0].w, d[0][1].x, d[0][1].y, d[0][1].z, d[0][1].w},
+                                    {d[1][0].x, d[1][0].y, d[1][0].z, d[1][0].w, d[1][1].x, d[1][1].y, d[1][1].z, d[1][1].w}};
+            float dist[8], out[8];
+            uint32_t kbest[8], best[8];
+            dist[0] = FLT_MAX;
+            kbest[0] = 0;
+            float all = FLT_MAX;  // over `width` slots
+            uint32_t kall = 0;
+#pragma unroll
+            for (int j = 2; j <= 8; ++j) {  // j slots shared by the two children
+                float b = FLT_MAX;
+                uint32_t bk = 1;
+#pragma unroll
+                for (int k = 1; k < j; ++k) {
+                    const float v = cc[0][k - 1] + cc[1][j - k - 1];
+                    if (v < b) {
+                        b = v;
+                        bk = k;
+                    }
+                }
+                dist[j - 1] = b;
+                kbest[j - 1] = bk;
+                if (j == width) {
+                    all = b;
+                    kall = bk;
+                }
+            }
+            const float leaf_cost = count <= kCwMaxLeaf ? kCwCostTri * a * (float)count : FLT_MAX;
+            const float node_cost = kCwCostNode * a + all;
+            const bool leaf = leaf_cost <= node_cost;
+            float v = leaf ? leaf_cost : node_cost;
+            out[0] = v;
+            best[0] = kall;
+#pragma unroll
+            for (int j = 2; j <= 8; ++j) {
+                const bool better = j <= width && dist[j - 1] < v;
+                if (better) v = dist[j - 1];
+                out[j - 1] = v;
+                best[j - 1] = better ? kbest[j - 1] : 0u;
+            }
+            float4* q = reinterpret_cast<float4*>(dp_cost + (size_t)p * 8);
+            q[0] = f4(out[0], out[1], out[2], out[3]);
+            q[1] = f4(out[4], out[5], out[6], out[7]);
+            *reinterpret_cast<uint2*>(dp_split + (size_t)p * 8) =
+                make_uint2(best[0] | best[1] << 8 | best[2] << 16 | best[3] << 24,
+                           best[4] | best[5] << 8 | best[6] << 16 | best[7] << 24);
+            cw_collapse[p] = leaf ? 1u : 0u;
+        }
         p = parent_i[p];
     }
 }
@@ -314,43 +407,84 @@ __global__ void init_bounds_kernel(uint32_t* cb) {
 
 inline uint32_t blocks(uint32_t n, uint32_t b = 256) { return (n + b - 1) / b; }
 
-// Allocates the scratch of one build (stream-ordered).
-cudaError_t scratch_alloc(Scratch& s, uint32_t n, cudaStream_t st) {
+// Lays the scratch of one build over n items out in the context's arena.
+cudaError_t scratch_carve(Scratch& s, uint32_t n, BuildArena& arena, cudaStream_t st) {
     std::memset(&s, 0, sizeof(s));
     const size_t m = n > 1 ? n - 1 : 1;
-    CK(cudaMallocAsync((void**)&s.lo, n * sizeof(float4), st));
-    CK(cudaMallocAsync((void**)&s.hi, n * sizeof(float4), st));
-    CK(cudaMallocAsync((void**)&s.morton_in, n * sizeof(uint32_t), st));
-    CK(cudaMallocAsync((void**)&s.morton, n * sizeof(uint32_t), st));
-    CK(cudaMallocAsync((void**)&s.idx_in, n * sizeof(uint32_t), st));
-    CK(cudaMallocAsync((void**)&s.idx, n * sizeof(uint32_t), st));
-    CK(cudaMallocAsync((void**)&s.left, m * sizeof(int32_t), st));
-    CK(cudaMallocAsync((void**)&s.right, m * sizeof(int32_t), st));
-    CK(cudaMallocAsync((void**)&s.parent_i, m * sizeof(int32_t), st));
-    CK(cudaMallocAsync((void**)&s.parent_l, n * sizeof(int32_t), st));
-    CK(cudaMallocAsync((void**)&s.range_lo, m * sizeof(uint32_t), st));
-    CK(cudaMallocAsync((void**)&s.range_hi, m * sizeof(uint32_t), st));
-    CK(cudaMallocAsync((void**)&s.ilo, m * sizeof(float4), st));
-    CK(cudaMallocAsync((void**)&s.ihi, m * sizeof(float4), st));
-    CK(cudaMallocAsync((void**)&s.cost, m * sizeof(float), st));
-    CK(cudaMallocAsync((void**)&s.collapse, m * sizeof(uint32_t), st));
-    CK(cudaMallocAsync((void**)&s.arrive, m * sizeof(uint32_t), st));
-    CK(cudaMallocAsync((void**)&s.cbounds, 8 * sizeof(uint32_t), st));
     CK(cub::DeviceRadixSort::SortPairs(nullptr, s.cub_bytes, s.morton_in, s.morton, s.idx_in, s.idx, (int)n, 0, 30,
                                        st));
-    CK(cudaMallocAsync(&s.cub_tmp, s.cub_bytes ? s.cub_bytes : 16, st));
+    for (int pass = 0; pass < 2; ++pass) {  // measure, then place
+        char* p = static_cast<char*>(arena.p);
+        size_t used = 0;
+        auto take = [&](auto*& ptr, size_t count) {
+            if (pass) ptr = reinterpret_cast<std::remove_reference_t<decltype(ptr)>>(p + used);
+            used += (count * sizeof(*ptr) + 255) & ~size_t(255);
+        };
+        take(s.lo, n);
+        take(s.hi, n);
+        take(s.morton_in, n);
+        take(s.morton, n);
+        take(s.idx_in, n);
+        take(s.idx, n);
+        take(s.left, m);
+        take(s.right, m);
+        take(s.parent_i, m);
+        take(s.parent_l, n);
+        take(s.range_lo, m);
+        take(s.range_hi, m);
+        take(s.cost, m);
+        take(s.collapse, m);
+        take(s.arrive, m);
+        take(s.cbounds, 8);
+        take(s.unsorted, n);
+        char* tmp = nullptr;
+        take(tmp, s.cub_bytes ? s.cub_bytes : 16);
+        s.cub_tmp = tmp;
+        take(s.dp_split, m * 8);
+        take(s.cw_collapse, m);
+        take(s.task_a, n);
+        take(s.task_b, n);
+        take(s.counters, 4);
+        for (int k = 0; k < 2; ++k) take(s.p_cid[k], n);
+        take(s.p_partner, n);
+        take(s.p_left, m);
+        take(s.p_right, m);
+        take(s.p_parent, m);
+        take(s.p_lparent, n);
+        take(s.p_cnt, m);
+        take(s.p_pre, m);
+        take(s.p_off, m);
+        take(s.p_loff, n);
+        take(s.p_tile, n / 256 + 1);
+        take(s.p_state, 8);
+        // clusters' boxes; after the clustering inner boxes and the collapse's costs
+        for (int k = 0; k < 2; ++k) {
+            take(s.p_lo[k], n);
+            take(s.p_hi[k], n);
+        }
+        s.ilo = s.p_lo[0];
+        s.ihi = s.p_hi[0];
+        s.dp_cost = reinterpret_cast<float*>(s.p_lo[1]);
+        if (!pass) CK(arena.reserve(used));
+    }
     return cudaSuccess;
 }
 
-void scratch_free(Scratch& s, cudaStream_t st) {
-    void* ptrs[] = {s.lo, s.hi, s.morton_in, s.morton, s.idx_in, s.idx, s.left, s.right, s.parent_i,
-                    s.parent_l, s.range_lo, s.range_hi, s.ilo, s.ihi, s.cost, s.collapse, s.arrive, s.cbounds,
-                    s.cub_tmp};
-    for (void* p : ptrs)
-        if (p) cudaFreeAsync(p, st);
-}
-
 }  // namespace
+
+cudaError_t BuildArena::reserve(size_t n) {
+    if (n <= bytes) return cudaSuccess;
+    release();
+    const cudaError_t e = cudaMalloc(&p, n);
+    if (e == cudaSuccess) bytes = n;
+    else p = nullptr;
+    return e;
+}
+void BuildArena::release() {
+    if (p) cudaFree(p);
+    p = nullptr;
+    bytes = 0;
+}
 
 #include "ploc_build.inc"
 
@@ -358,11 +492,9 @@ namespace {
 
 // Morton codes, sort, binary tree (PLOC clustering, or the Karras radix tree
 // when quality is kBvhFast) and the bottom-up pass (boxes, SAH costs, leaf
-// collapse with at most max_leaf items, an inner node costing cost_traverse
-// triangle tests per unit of area).  Item boxes in s.lo/hi and centroid
-// bounds in s.cbounds must be ready.
-cudaError_t radix_tree(Scratch& s, uint32_t n, uint32_t max_leaf, cudaStream_t st, int quality,
-                       float cost_traverse = kCostTraverse) {
+// collapse; for width > 0 also the wide collapse's distribution).  Item boxes
+// in s.lo/hi and centroid bounds in s.cbounds must be ready.
+cudaError_t binary_tree(Scratch& s, uint32_t n, cudaStream_t st, int quality, int width) {
     morton_kernel<<<blocks(n), 256, 0, st>>>(s.lo, s.hi, n, s.cbounds, s.morton_in, s.idx_in);
     CK(cudaGetLastError());
     CK(cub::DeviceRadixSort::SortPairs(s.cub_tmp, s.cub_bytes, s.morton_in, s.morton, s.idx_in, s.idx, (int)n, 0,
@@ -376,18 +508,25 @@ cudaError_t radix_tree(Scratch& s, uint32_t n, uint32_t max_leaf, cudaStream_t s
             CK(cudaGetLastError());
         }
         CK(cudaMemsetAsync(s.arrive, 0, (n - 1) * sizeof(uint32_t), st));
-        bottom_up_kernel<<<blocks(n), 256, 0, st>>>((int)n, s.idx, s.lo, s.hi, s.left, s.right, s.parent_i,
-                                                   s.parent_l, s.range_lo, s.range_hi, s.ilo, s.ihi, s.cost,
-                                                   s.collapse, s.arrive, max_leaf, cost_traverse);
+        if (width)
+            bottom_up_kernel<true><<<blocks(n), 256, 0, st>>>((int)n, s.idx, s.lo, s.hi, s.left, s.right, s.parent_i,
+                                                              s.parent_l, s.range_lo, s.range_hi, s.ilo, s.ihi, s.cost,
+                                                              s.collapse, s.arrive, s.dp_cost, s.dp_split,
+                                                              s.cw_collapse, width);
+        else
+            bottom_up_kernel<false><<<blocks(n), 256, 0, st>>>((int)n, s.idx, s.lo, s.hi, s.left, s.right, s.parent_i,
+                                                               s.parent_l, s.range_lo, s.range_hi, s.ilo, s.ihi,
+                                                               s.cost, s.collapse, s.arrive, nullptr, nullptr,
+                                                               nullptr, 0);
         CK(cudaGetLastError());
     }
     return cudaSuccess;
 }
 
-// Common tail: radix tree with leaves of up to kMaxLeaf items, emit BNode2.
+// Common tail: binary tree with leaves of up to kMaxLeaf items, emit BNode2.
 cudaError_t build_common(Scratch& s, uint32_t n, BNode2* nodes, uint32_t node_base, uint32_t tri_base,
-                         BvhResult* res, cudaStream_t st, int quality) {
-    CK(radix_tree(s, n, kMaxLeaf, st, quality));
+                         BvhResult* res, cudaStream_t st, int quality, int width = 0) {
+    CK(binary_tree(s, n, st, quality, width));
     if (n > 1) {
         emit_nodes_kernel<<<blocks(n - 1), 256, 0, st>>>((int)n, s.idx, s.lo, s.hi, s.left, s.right, s.range_lo,
                                                         s.range_hi, s.ilo, s.ihi, s.collapse, nodes, node_base,
@@ -416,51 +555,39 @@ cudaError_t build_common(Scratch& s, uint32_t n, BNode2* nodes, uint32_t node_ba
 
 }  // namespace
 
-cudaError_t build_triangle_bvh(const gbrt_vertex* vertices, const uint32_t* indices, const gbrt_priminfo* prims,
-                               const uint4* items, uint32_t n, BNode2* nodes, uint32_t node_base, TriRec* tris,
-                               uint32_t tri_base, BvhResult* res, cudaStream_t st, const DevInstance* inst,
-                               int quality) {
-    if (n == 0) return cudaErrorInvalidValue;
+#include "cwbvh_build.inc"
+
+cudaError_t build_triangle_bvh(BuildArena& arena, const gbrt_vertex* vertices, const uint32_t* indices,
+                               const gbrt_priminfo* prims, const uint4* items, uint32_t n, BNode2* nodes,
+                               uint32_t node_base, TriRec* tris, uint32_t tri_base, BvhResult* res, cudaStream_t st,
+                               const DevInstance* inst, int quality, const WideBuild* wide) {
+    if (n == 0 || (wide && (wide->width < 2 || wide->width > 8))) return cudaErrorInvalidValue;
     Scratch s;
-    cudaError_t e = scratch_alloc(s, n, st);
-    TriRec* unsorted = nullptr;
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&unsorted, n * sizeof(TriRec), st);
-    if (e == cudaSuccess) {
-        init_bounds_kernel<<<1, 32, 0, st>>>(s.cbounds);
-        tri_boxes_kernel<<<blocks(n), 256, 0, st>>>(vertices, indices, prims, items, n, s.lo, s.hi, unsorted,
-                                                    s.cbounds, inst);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = build_common(s, n, nodes, node_base, tri_base, res, st, quality);
-    if (e == cudaSuccess) {
-        gather_tris_kernel<<<blocks(n), 256, 0, st>>>(s.idx, n, unsorted, tris, tri_base);
-        e = cudaGetLastError();
-    }
-    if (unsorted) cudaFreeAsync(unsorted, st);
-    scratch_free(s, st);
-    return e;
+    CK(scratch_carve(s, n, arena, st));
+    init_bounds_kernel<<<1, 32, 0, st>>>(s.cbounds);
+    tri_boxes_kernel<<<blocks(n), 256, 0, st>>>(vertices, indices, prims, items, n, s.lo, s.hi, s.unsorted, s.cbounds,
+                                                inst);
+    CK(cudaGetLastError());
+    CK(build_common(s, n, nodes, node_base, tri_base, res, st, quality, wide ? wide->width : 0));
+    gather_tris_kernel<<<blocks(n), 256, 0, st>>>(s.idx, n, s.unsorted, tris, tri_base);
+    CK(cudaGetLastError());
+    return wide ? emit_wide(s, n, *wide, st) : cudaSuccess;
 }
 
-cudaError_t build_instance_bvh(const float4* lo, const float4* hi, const uint32_t* ids, uint32_t n, BNode2* nodes,
-                               uint32_t node_base, TriRec* tris, uint32_t tri_base, BvhResult* res,
+cudaError_t build_instance_bvh(BuildArena& arena, const float4* lo, const float4* hi, const uint32_t* ids, uint32_t n,
+                               BNode2* nodes, uint32_t node_base, TriRec* tris, uint32_t tri_base, BvhResult* res,
                                cudaStream_t st, int quality) {
     if (n == 0) return cudaErrorInvalidValue;
     Scratch s;
-    cudaError_t e = scratch_alloc(s, n, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(s.lo, lo, n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(s.hi, hi, n * sizeof(float4), cudaMemcpyDeviceToDevice, st);
-    if (e == cudaSuccess) {
-        init_bounds_kernel<<<1, 32, 0, st>>>(s.cbounds);
-        box_centroid_bounds_kernel<<<blocks(n), 256, 0, st>>>(s.lo, s.hi, n, s.cbounds);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = build_common(s, n, nodes, node_base, tri_base, res, st, quality);
-    if (e == cudaSuccess) {
-        gather_inst_kernel<<<blocks(n), 256, 0, st>>>(s.idx, n, ids, tris, tri_base);
-        e = cudaGetLastError();
-    }
-    scratch_free(s, st);
-    return e;
+    CK(scratch_carve(s, n, arena, st));
+    CK(cudaMemcpyAsync(s.lo, lo, n * sizeof(float4), cudaMemcpyDeviceToDevice, st));
+    CK(cudaMemcpyAsync(s.hi, hi, n * sizeof(float4), cudaMemcpyDeviceToDevice, st));
+    init_bounds_kernel<<<1, 32, 0, st>>>(s.cbounds);
+    box_centroid_bounds_kernel<<<blocks(n), 256, 0, st>>>(s.lo, s.hi, n, s.cbounds);
+    CK(cudaGetLastError());
+    CK(build_common(s, n, nodes, node_base, tri_base, res, st, quality));
+    gather_inst_kernel<<<blocks(n), 256, 0, st>>>(s.idx, n, ids, tris, tri_base);
+    return cudaGetLastError();
 }
 
 size_t bvh_sort_temp_bytes(uint32_t n) {
@@ -589,8 +716,4 @@ cudaError_t instance_world_boxes(const DevInstance* inst, const uint32_t* ids, c
     return cudaGetLastError();
 }
 
-}  // namespace gbrt
-
-namespace gbrt {
-#include "cwbvh_build.inc"
 }  // namespace gbrt

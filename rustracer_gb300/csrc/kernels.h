@@ -200,14 +200,44 @@ struct BvhResult {
 // round), kBvhFast splits the Morton order (Karras radix tree, one launch).
 constexpr int kBvhFast = 0, kBvhPloc = 1;
 
+// Device memory that the builds of a context carve their scratch from: grown
+// to the largest build's need (about 270 B per triangle) and kept, so that a
+// rebuild of an animated scene does not allocate.  One build at a time uses
+// it, in the order of the context's stream.
+struct BuildArena {
+    void* p = nullptr;
+    size_t bytes = 0;
+    BuildArena() = default;
+    BuildArena(const BuildArena&) = delete;
+    BuildArena& operator=(const BuildArena&) = delete;
+    ~BuildArena() { release(); }
+    cudaError_t reserve(size_t n);
+    void release();
+};
+
+// The compressed 8-wide form of a triangle BVH, built from the same binary
+// tree: nodes (capacity n, root at 0) and their triangles (n slots, node-leaf
+// order); *nodes_used gets the node count, level_starts (may be null) the
+// first node of each level and the node count.  width 4 collapses to at most
+// 4 children per node (same node format, so the same traversal).
+struct WideBuild {
+    CwNode* nodes;
+    TriRec* tris;
+    uint32_t* nodes_used;
+    std::vector<uint32_t>* level_starts;
+    int width;
+};
+
 // Item descriptors for triangle BVHs: x = instance id (world BVH) or 0,
 // y = BLAS geometry id, z = primitive id, w = opaque flag.
 // inst (may be null): items whose instance is not an identity one are
-// transformed to world space (flattened instances).
-cudaError_t build_triangle_bvh(const gbrt_vertex* vertices, const uint32_t* indices, const gbrt_priminfo* prims,
-                               const uint4* items, uint32_t n, BNode2* nodes, uint32_t node_base, TriRec* tris,
-                               uint32_t tri_base, BvhResult* result_host, cudaStream_t st,
-                               const DevInstance* inst = nullptr, int quality = kBvhPloc);
+// transformed to world space (flattened instances).  wide (may be null): the
+// 8-wide form is built as well.
+cudaError_t build_triangle_bvh(BuildArena& arena, const gbrt_vertex* vertices, const uint32_t* indices,
+                               const gbrt_priminfo* prims, const uint4* items, uint32_t n, BNode2* nodes,
+                               uint32_t node_base, TriRec* tris, uint32_t tri_base, BvhResult* result_host,
+                               cudaStream_t st, const DevInstance* inst = nullptr, int quality = kBvhPloc,
+                               const WideBuild* wide = nullptr);
 
 // Scratch of one triangle-BVH build supplied by the caller instead of being
 // allocated (every pointer 256-byte aligned, sized for `capacity` items).
@@ -236,15 +266,7 @@ cudaError_t build_triangle_bvh_scratch(const BuildScratch& scratch, const gbrt_v
                                        uint32_t n, BNode2* nodes, uint32_t node_base, TriRec* tris,
                                        uint32_t tri_base, BvhResult* result_host, cudaStream_t st);
 
-// Compressed 8-wide BVH over n triangle items: nodes (capacity n, root at 0)
-// and their triangles (n slots, node-leaf order); *nodes_used (host) gets
-// the node count.  width 4 collapses to at most 4 children per node (same
-// node format, so the same traversal).
-cudaError_t build_triangle_cwbvh(const gbrt_vertex* vertices, const uint32_t* indices, const gbrt_priminfo* prims,
-                                 const uint4* items, uint32_t n, CwNode* nodes, TriRec* tris, uint32_t* nodes_used,
-                                 cudaStream_t st, std::vector<uint32_t>* level_starts = nullptr,
-                                 const DevInstance* inst = nullptr, int width = 8, int quality = kBvhPloc);
-// Refit of an 8-wide BVH built by build_triangle_cwbvh over the same
+// Refit of an 8-wide BVH built by build_triangle_bvh over the same
 // triangles: triangle records re-read from the vertices, then every node's
 // grid and child boxes recomputed level by level (level_starts: first node
 // of each level, last entry = node count).  boxes: scratch of 2 float4 per
@@ -259,16 +281,9 @@ cudaError_t refit_triangle_cwbvh(const gbrt_vertex* vertices, const uint32_t* in
 
 // TLAS over instances: boxes given per instance (lo/hi), the leaf slots carry
 // the instance ids.
-cudaError_t build_instance_bvh(const float4* lo, const float4* hi, const uint32_t* inst_ids, uint32_t n,
+cudaError_t build_instance_bvh(BuildArena& arena, const float4* lo, const float4* hi, const uint32_t* inst_ids, uint32_t n,
                                BNode2* nodes, uint32_t node_base, TriRec* tris, uint32_t tri_base,
                                BvhResult* result_host, cudaStream_t st, int quality = kBvhPloc);
-
-// Refit: recomputes every inner-node box of a triangle BVH bottom-up from the
-// current vertex positions, keeping the topology (used after skinning).
-cudaError_t refit_triangle_bvh(const gbrt_vertex* vertices, const uint32_t* indices, const gbrt_priminfo* prims,
-                               BNode2* nodes, uint32_t node_base, uint32_t num_inner, TriRec* tris,
-                               uint32_t tri_base, uint32_t n, const int32_t* parents, int32_t root,
-                               BvhResult* result_host, cudaStream_t st);
 
 // World boxes of transformed instances from their BLAS root bounds.
 cudaError_t instance_world_boxes(const DevInstance* inst, const uint32_t* ids, const float4* blas_lo,
