@@ -272,7 +272,8 @@ int build_all(gbrt_scene* s) {
         const size_t nw = world_items.size();
         CU(c, s->cw_nodes.alloc(nw * sizeof(CwNode)), "cudaMalloc(wide nodes)");
         CU(c, s->cw_tris.alloc(nw * sizeof(TriRec)), "cudaMalloc(wide triangles)");
-        const WideBuild wide{s->cw_nodes.as<CwNode>(), s->cw_tris.as<TriRec>(), &s->cw_count, &s->cw_levels, cw_width(s)};
+        const WideBuild wide{s->cw_nodes.as<CwNode>(), s->cw_tris.as<TriRec>(), &s->cw_count, &s->cw_levels, cw_width(s),
+                             &s->cw_sah0};
         CU(c, build_triangle_bvh(c->build, s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
                                  s->prims.as<gbrt_priminfo>(), s->items.as<uint4>(), (uint32_t)nw,
                                  s->nodes.as<BNode2>(), 0, s->tris.as<TriRec>(), 0, &r, st, s->inst.as<DevInstance>(),
@@ -283,19 +284,10 @@ int build_all(gbrt_scene* s) {
         v.world_lo = r.lo;
         v.world_hi = r.hi;
         s->nworld = (uint32_t)nw;
-        // the tree's SAH cost proxy as built (a refit of unchanged vertices rewrites the same nodes), the
-        // reference for the drift check of later refits
-        s->cw_sah0 = 0.0;
+        // the SAH cost proxy as built is the reference for the drift check of later refits
+        s->cw_sah = s->cw_sah0;
         s->refits = 0;
-        if (s->cw_levels.size() >= 2) {
-            CU(c, s->cw_boxes.reserve((size_t)s->cw_count * 2 * sizeof(float4) + 16), "cudaMalloc(refit boxes)");
-            CU(c, refit_triangle_cwbvh(s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
-                                       s->prims.as<gbrt_priminfo>(), s->cw_nodes.as<CwNode>(), s->cw_tris.as<TriRec>(),
-                                       s->nworld, s->cw_levels, s->cw_boxes.as<float4>(), st,
-                                       s->inst.as<DevInstance>(), &s->cw_sah0),
-               "measure wide world BVH");
-            s->cw_sah = s->cw_sah0;
-        }
+        CU(c, s->cw_boxes.reserve((size_t)s->cw_count * 2 * sizeof(float4) + 16), "cudaMalloc(refit boxes)");
     } else {
         s->cw_nodes.release();
         s->cw_tris.release();
@@ -327,7 +319,7 @@ int build_all(gbrt_scene* s) {
             BvhResult r;
             uint32_t used = 0;
             const WideBuild wide{s->blas_cw_nodes.as<CwNode>() + cw_node0[g], s->blas_cw_tris.as<TriRec>() + cw_tri0[g],
-                                 &used, nullptr, cw_width(s)};
+                                 &used, nullptr, cw_width(s), nullptr};
             CU(c, build_triangle_bvh(c->build, s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
                                      s->prims.as<gbrt_priminfo>(), bitems.as<uint4>(), ntri, s->nodes.as<BNode2>(),
                                      blas_node_base[g], s->tris.as<TriRec>(), blas_tri_base[g], &r, st, nullptr,

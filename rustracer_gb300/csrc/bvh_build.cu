@@ -11,6 +11,7 @@
 // written in the traversal layout (BNode2 with both child boxes; leaves as
 // codes over a contiguous range of TriRec slots in Morton order).
 #include <cub/device/device_radix_sort.cuh>
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <utility>
@@ -70,7 +71,8 @@ struct Scratch {
     float* dp_cost;         // [n-1][8]
     uint8_t* dp_split;      // [n-1][8]
     uint32_t* cw_collapse;  // [n-1] 1 = one leaf slot of a wide node
-    uint2 *task_a, *task_b; // [n]
+    int32_t* cw_task;       // [n] binary node of each wide node
+    uint2* cw_level;        // [n + 16] first node and node count of each level
     uint32_t* counters;     // 4
     // clustering (ploc_build.inc); the boxes share memory with what is written after it
     int32_t* p_cid[2];
@@ -442,8 +444,8 @@ cudaError_t scratch_carve(Scratch& s, uint32_t n, BuildArena& arena, cudaStream_
         s.cub_tmp = tmp;
         take(s.dp_split, m * 8);
         take(s.cw_collapse, m);
-        take(s.task_a, n);
-        take(s.task_b, n);
+        take(s.cw_task, n);
+        take(s.cw_level, (size_t)n + 16);
         take(s.counters, 4);
         for (int k = 0; k < 2; ++k) take(s.p_cid[k], n);
         take(s.p_partner, n);
@@ -571,7 +573,7 @@ cudaError_t build_triangle_bvh(BuildArena& arena, const gbrt_vertex* vertices, c
     CK(build_common(s, n, nodes, node_base, tri_base, res, st, quality, wide ? wide->width : 0));
     gather_tris_kernel<<<blocks(n), 256, 0, st>>>(s.idx, n, s.unsorted, tris, tri_base);
     CK(cudaGetLastError());
-    return wide ? emit_wide(s, n, *wide, st) : cudaSuccess;
+    return wide ? emit_wide(s, n, *wide, *res, st) : cudaSuccess;
 }
 
 cudaError_t build_instance_bvh(BuildArena& arena, const float4* lo, const float4* hi, const uint32_t* ids, uint32_t n,

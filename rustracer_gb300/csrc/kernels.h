@@ -218,14 +218,16 @@ struct BuildArena {
 // The compressed 8-wide form of a triangle BVH, built from the same binary
 // tree: nodes (capacity n, root at 0) and their triangles (n slots, node-leaf
 // order); *nodes_used gets the node count, level_starts (may be null) the
-// first node of each level and the node count.  width 4 collapses to at most
-// 4 children per node (same node format, so the same traversal).
+// first node of each level and the node count, *sah (may be null) the tree's
+// SAH cost proxy (refit_triangle_cwbvh).  width 4 collapses to at most 4
+// children per node (same node format, so the same traversal).
 struct WideBuild {
     CwNode* nodes;
     TriRec* tris;
     uint32_t* nodes_used;
     std::vector<uint32_t>* level_starts;
     int width;
+    double* sah;
 };
 
 // Item descriptors for triangle BVHs: x = instance id (world BVH) or 0,
