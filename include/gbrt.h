@@ -244,7 +244,8 @@ typedef struct gbrt_stats {
     double   device_ms;       /* CUDA-event time of the device work */
     uint32_t kernel_launches;
     uint32_t device_status;   /* 0, or GBRT_STATUS_* bits reported by kernels */
-    uint64_t node_visits;     /* BVH inner nodes visited by all traversals */
+    uint64_t node_visits;     /* BVH inner nodes visited by all traversals (varies by a few
+                                 percent between runs, as lanes share long rays) */
     uint64_t tri_tests;       /* ray-triangle tests */
     double   stage_ms[4];     /* with GBRT_RENDER_STAGE_TIMING (wavefront form):
                                  extend, shade, shadow, other kernels */

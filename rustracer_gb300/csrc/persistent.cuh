@@ -227,8 +227,13 @@ GB_D uint32_t warp_scan(uint32_t v) {
 struct WarpTris {
     float4 o[32];     // origin, tmin
     float4 s[32];     // shear constants, axis permutation kx | ky << 2 | kz << 4
-    uint2 pair[32];   // triangle slot, lane of its ray
+    uint2 pair[32];   // triangle slot, lane of its ray; or work handed to an idle lane
+    uint32_t helpers[32];  // lanes that work on this lane's ray besides itself
 };
+
+// Idle lanes of a warp that make it worth handing work out (2, 8 and 16 measure
+// the same within 2%).
+constexpr int kSteal = 8;
 
 // Persistent-lane traversal of the 8-wide world BVH; same interface and
 // refill policy as persistent_trace.
@@ -240,13 +245,27 @@ struct WarpTris {
 // lane with the most triangles finished.  The owner of a ray then takes the
 // results of its triangles in slot order, so hits are those of the
 // lane-by-lane loop.  Icosphere frame (1080p x 64): extend 41.5 -> 36.7 ms,
-// shadow 22.4 -> 18.0; 1.5M incoherent ray queries 383 -> 310 us.  kHit: the finisher reads the hit
-// of an any-hit query, not only whether there is one.  Every block has at
-// most 128 threads.
+// shadow 22.4 -> 18.0; 1.5M incoherent ray queries 383 -> 310 us.
+//
+// Once the queue is empty (exhausted), idle lanes take subtrees from lanes
+// that have some pending, with a copy of the ray: a launch ends with its
+// longest rays, whose dozens of steps in a row took most of the time of waves
+// of up to a million rays while the rest of the GPU was idle.  A helper hands
+// every hit to the ray's owner, which settles ties as ever and reports once
+// nobody works on its ray (WarpTris::helpers), so hits do not depend on who
+// helps; the statistics' node and triangle counts do, by a few percent.  64 x
+// 64 frames of instanced tori 820 -> 519 us, of an icosphere 348 -> 301, 854 x
+// 480 x 3 viewer 1.10 -> 1.00 ms; 1080p x 64 icosphere 77.0 -> 77.3.
+//
+// kHit: the finisher reads the hit of an any-hit query, not only whether there
+// is one; such a query takes no help, so that it reports the first hit of the
+// traversal order whatever its neighbours do.  Every block has at most 128
+// threads.
 template <bool kAny, bool kTlas, bool kAlpha, bool kHit, class Loader, class Finisher>
 GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uint32_t flags, TraceStats& ts,
                               uint32_t quota, Loader&& load, Finisher&& finish) {
     constexpr uint32_t kAll = 0xFFFFFFFFu, kInner = 0xFF000000u;
+    constexpr bool kHelp = !(kAny && kHit);
     __shared__ WarpTris s_tris[4];
     WarpTris& sw = s_tris[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
@@ -260,7 +279,9 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
     float tmin = 0.0f, tmax = 0.0f;
     uint2 ng = make_uint2(0, 0);
     int sp = 0;
+    uint32_t own = lane;  // the lane whose ray this one works on (itself until idle lanes help)
     uint32_t iter = 0;
+    if (kHelp) sw.helpers[lane] = 0u;
     for (;;) {
         if (!exhausted) {
             const uint32_t idle = __ballot_sync(kAll, !has);
@@ -300,6 +321,61 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
         if (!__any_sync(kAll, has)) {
             if (exhausted) break;
             continue;
+        }
+        // --- no more rays: idle lanes take work from busy ones ------------------
+        if (kHelp && exhausted) {
+            const uint32_t idle = __ballot_sync(kAll, !has), inner = ng.y & kInner;
+            const bool rich = has && (sp > 0 || (inner & (inner - 1u)));
+            const uint32_t donors = __ballot_sync(kAll, rich);
+            const int pairs = min(__popc(idle), __popc(donors)), rank = __popc((rich ? donors : idle) & ((1u << lane) - 1u));
+            if (pairs && __popc(idle) >= kSteal) {
+                if (rich && rank < pairs) {  // the last stack entry, or all but the next child; bits 8..12: from whom
+                    uint2 give;
+                    if (sp > 0) {
+                        give = stack[--sp];
+                    } else {
+                        give = make_uint2(ng.x, ng.y & ~(inner & (0u - inner)));
+                        ng.y = (inner & (0u - inner)) | (ng.y & 0xFFu);
+                    }
+                    sw.pair[rank] = make_uint2(give.x, give.y | lane << 8);
+                }
+                __syncwarp();
+                const bool take = !has && rank < pairs;
+                uint2 got = make_uint2(0u, lane << 8);
+                if (take) got = sw.pair[rank];
+                const uint32_t from = (got.y >> 8) & 31u;
+                const float ix = __shfl_sync(kAll, r.inv.x, from), iy = __shfl_sync(kAll, r.inv.y, from),
+                            iz = __shfl_sync(kAll, r.inv.z, from), bt = __shfl_sync(kAll, best.t, from);
+                const uint32_t o2 = __shfl_sync(kAll, oct, from), w2 = __shfl_sync(kAll, own, from);
+                AnyCtx c2{0, 0, 0, 0};
+                if constexpr (kAlpha)
+                    c2 = AnyCtx{__shfl_sync(kAll, ctx.px, from), __shfl_sync(kAll, ctx.py, from),
+                                __shfl_sync(kAll, ctx.sample, from), __shfl_sync(kAll, ctx.tag, from)};
+                if (take) {
+                    const float4 o4 = sw.o[from];
+                    sw.o[lane] = o4;
+                    sw.s[lane] = sw.s[from];
+                    r.o = f3(o4);
+                    r.inv = f3(ix, iy, iz);
+                    tmin = o4.w;
+                    oct = o2;
+                    own = w2;
+                    if constexpr (kAlpha) ctx = c2;
+                    best.t = bt;
+                    best.inst = best.prim = 0xFFFFFFFFu;
+                    ng = make_uint2(got.x, got.y & (kInner | 0xFFu));
+                    sp = 0;
+                    iter = 0;
+                    has = true;
+                    atomicAdd(&sw.helpers[own], 1u);
+                }
+                __syncwarp();
+            }
+            const float ot = __shfl_sync(kAll, best.t, own);
+            if (own != lane && ot < best.t) {  // ties with the owner's hit are settled by the owner
+                best.t = ot;
+                best.inst = best.prim = 0xFFFFFFFFu;
+            }
         }
         // --- one node per ray -------------------------------------------------
         bool done = false;
@@ -396,7 +472,15 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
                     best.inst = 0u;
                 }
                 done = done || my;
+                if constexpr (kHelp) {
+                    if (exhausted) {
+                        uint32_t up = __ballot_sync(kAll, my && own != lane);  // helpers' hits end their owners' rays
+                        for (; up; up &= up - 1u)
+                            if (lane == __shfl_sync(kAll, own, __ffs(up) - 1)) best.inst = 0u;
+                    }
+                }
             } else {
+                bool fresh = false;
                 while (__any_sync(kAll, my != 0u)) {
                     const uint32_t f = my ? __ffs(my) - 1u : lane;
                     const float t2 = __shfl_sync(kAll, t, f), u2 = __shfl_sync(kAll, u, f),
@@ -408,12 +492,41 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
                         best.v = v2;
                         best.inst = i2;
                         best.prim = p2;
+                        fresh = true;
                     }
                     my &= my - 1u;
                 }
+                if constexpr (kHelp) {
+                    if (exhausted) {  // helpers' hits go to their owners at once
+                        for (uint32_t up = __ballot_sync(kAll, fresh && own != lane); up; up &= up - 1u) {
+                            const int f = __ffs(up) - 1;
+                            const float t2 = __shfl_sync(kAll, best.t, f), u2 = __shfl_sync(kAll, best.u, f),
+                                        v2 = __shfl_sync(kAll, best.v, f);
+                            const uint32_t i2 = __shfl_sync(kAll, best.inst, f), p2 = __shfl_sync(kAll, best.prim, f);
+                            if (lane == __shfl_sync(kAll, own, f) && closer(t2, i2, p2, best)) {
+                                best.t = t2;
+                                best.u = u2;
+                                best.v = v2;
+                                best.inst = i2;
+                                best.prim = p2;
+                            }
+                        }
+                    }
+                }
             }
         }
-        if (has && (done || (!(ng.y & kInner) && sp == 0))) {
+        bool last = true;  // nobody else works on this ray
+        if (kHelp && exhausted) {
+            const uint32_t found = __shfl_sync(kAll, best.inst, own);  // by every lane, done or not
+            if (kAny && found != 0xFFFFFFFFu) done = true;
+            if (has && own != lane && (done || (!(ng.y & kInner) && sp == 0))) {
+                has = false;
+                atomicSub(&sw.helpers[own], 1u);
+            }
+            __syncwarp();
+            last = own == lane && sw.helpers[lane] == 0u;
+        }
+        if (has && (done || (!(ng.y & kInner) && sp == 0)) && last) {
             if constexpr (kTlas) {
                 if (s.has_tlas && !(kAny && best.inst != 0xFFFFFFFFu))
                     trace_tlas<kAny, true>(s, r, r.o, r.d, tmin, best, test_alpha, ctx, ts);
