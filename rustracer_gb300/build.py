@@ -26,7 +26,7 @@ NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "--expt-relaxed-constexpr
 # with the explicit IEEE intrinsics (__fdiv_rn, __fsqrt_rn), which these flags
 # do not touch.
 SHADING_FLAGS = ["-prec-div=false", "-prec-sqrt=false"]
-SHADING_UNITS = {"wavefront.cu", "wave_multi.cu", "render.cu"}
+SHADING_UNITS = {"wavefront.cu", "shade_full.cu", "wave_multi.cu", "render.cu"}
 
 
 def nvcc():

@@ -535,14 +535,17 @@ int gbrt_ctx_create(int device, gbrt_ctx** out) {
     if ((e = cudaEventCreate(&c->tb1)) != cudaSuccess) return bail(e, "event");
     if ((e = c->counters.alloc(sizeof(DeviceCounters))) != cudaSuccess) return bail(e, "counters");
     if ((e = c->trace_work.alloc(256)) != cudaSuccess) return bail(e, "counters");
-    float lut[256];
+    float lut[512];  // sRGB-decoded, then linear 8-bit values
     for (int i = 0; i < 256; ++i) {
         double v = i / 255.0;
         lut[i] = (float)(v <= 0.04045 ? v / 12.92 : std::pow((v + 0.055) / 1.055, 2.4));
+        lut[256 + i] = (float)i / 255.0f;
     }
     if ((e = init_render_constants(lut)) != cudaSuccess) return bail(e, "constants");
     if ((e = init_wavefront_constants(lut)) != cudaSuccess) return bail(e, "constants");
     if ((e = init_wave_multi_constants(lut)) != cudaSuccess) return bail(e, "constants");
+    if ((e = init_rays_constants(lut)) != cudaSuccess) return bail(e, "constants");
+    if ((e = init_shade_full_constants(lut)) != cudaSuccess) return bail(e, "constants");
     *out = c;
     return GBRT_OK;
 }

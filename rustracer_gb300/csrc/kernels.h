@@ -146,8 +146,10 @@ struct StageTimer {
     int capacity = 0, used = 0;
 };
 size_t wavefront_bytes_per_path();
-cudaError_t init_wavefront_constants(const float* srgb_lut);
-cudaError_t init_wave_multi_constants(const float* srgb_lut);
+cudaError_t init_wavefront_constants(const float* texel_lut);
+cudaError_t init_wave_multi_constants(const float* texel_lut);
+cudaError_t init_rays_constants(const float* texel_lut);
+cudaError_t init_shade_full_constants(const float* texel_lut);
 // Grows a timer to hold `pairs` event pairs, keeping the pairs recorded so far.
 cudaError_t stage_timer_reserve(StageTimer& t, int pairs);
 // Fills the per-stage block partition of `w` (blocks in proportion to each
@@ -180,7 +182,7 @@ cudaError_t stage_timer_collect(StageTimer& t, double ms[4]);
 void stage_timer_free(StageTimer& t);
 
 // render.cu
-cudaError_t init_render_constants(const float* srgb_lut);
+cudaError_t init_render_constants(const float* texel_lut);
 cudaError_t launch_megakernel(const DevScene& s, const gbrt_ubo& ubo, const RenderOut& out, cudaStream_t st);
 cudaError_t launch_trace_rays(const DevScene& s, const gbrt_ray* rays, uint32_t n, uint32_t flags, gbrt_hit* hits,
                               DeviceCounters* cnt, cudaStream_t st);

@@ -34,6 +34,10 @@ __global__ void __launch_bounds__(128) trace_rays_persistent(DevScene s, const g
     if (cnt) flush_trace_stats(ts, cnt);
 }
 
+cudaError_t init_rays_constants(const float* texel_lut) {
+    return cudaMemcpyToSymbol(g_texel_lut, texel_lut, 512 * sizeof(float));
+}
+
 cudaError_t launch_trace_rays_persistent(const DevScene& s, const gbrt_ray* rays, uint32_t n, uint32_t flags,
                                          gbrt_hit* hits, uint32_t* work, DeviceCounters* cnt, cudaStream_t st) {
     if (n == 0) return cudaSuccess;

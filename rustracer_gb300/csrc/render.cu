@@ -166,8 +166,8 @@ __global__ void __launch_bounds__(128) trace_rays_kernel(DevScene s, const gbrt_
 }
 
 // --- host launchers --------------------------------------------------------
-cudaError_t init_render_constants(const float* srgb_lut) {
-    return cudaMemcpyToSymbol(c_srgb_lut, srgb_lut, 256 * sizeof(float));
+cudaError_t init_render_constants(const float* texel_lut) {
+    return cudaMemcpyToSymbol(g_texel_lut, texel_lut, 512 * sizeof(float));
 }
 
 cudaError_t launch_megakernel(const DevScene& s, const gbrt_ubo& ubo, const RenderOut& out, cudaStream_t st) {

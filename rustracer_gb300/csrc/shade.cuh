@@ -117,10 +117,19 @@ struct BrdfData {  // PBR.glsl:13-45
     bool Vbackfacing, Lbackfacing;
 };
 
+// x^5 of the Fresnel terms.  Units of shade kernels with every material feature
+// (GBRT_FULL_SHADE) call it: eight copies in line are part of what makes those
+// kernels wait for instructions (materials frame: shade 1.42 -> 1.25 ms), while
+// the plain kernel is better off with them (29.1 against 30.0 ms).
+#ifdef GBRT_FULL_SHADE
+static __device__ __noinline__ float pow5(float x) { return powf(x, 5.0f); }
+#else
+GB_D float pow5(float x) { return powf(x, 5.0f); }
+#endif
 GB_D float schlick(float cosine, float refractionIndex) {  // PBR.glsl:48-53
     float r0 = (1.0f - refractionIndex) / (1.0f + refractionIndex);
     r0 *= r0;
-    return r0 + (1.0f - r0) * powf(1.0f - cosine, 5.0f);
+    return r0 + (1.0f - r0) * pow5(1.0f - cosine);
 }
 GB_D void mat_build(MatBrdf& m) {  // matBuild, PBR.glsl:195-206
     float factor = (m.ior - 1.0f) / (m.ior + 1.0f);
@@ -132,7 +141,7 @@ GB_D void mat_build(MatBrdf& m) {  // matBuild, PBR.glsl:195-206
 }
 GB_D float saturatef(float x) { return clampf(x, 0.0f, 1.0f); }
 GB_D float3 fresnel(float3 f0, float f90, float NdotS) {  // evalFresnelSchlick, :228-231
-    return f0 + (f90 - f0) * powf(1.0f - NdotS, 5.0f);
+    return f0 + (f90 - f0) * pow5(1.0f - NdotS);
 }
 GB_D float smith_g_a(float alpha, float NdotS) {  // :248-250
     return NdotS / (fmaxf(0.00001f, alpha) * sqrtf(1.0f - fminf(0.99999f, NdotS * NdotS)));
@@ -202,8 +211,8 @@ GB_D float frostbite_diffuse(const BrdfData& d) {  // frostbiteDisneyDiffuse, :4
     float energyBias = 0.5f * d.roughness;
     float energyFactor = mixf(1.0f, 1.0f / 1.51f, d.roughness);
     float FD90MinusOne = energyBias + 2.0f * d.LdotH * d.LdotH * d.roughness - 1.0f;
-    float FDL = 1.0f + (FD90MinusOne * powf(1.0f - d.NdotL, 5.0f));
-    float FDV = 1.0f + (FD90MinusOne * powf(1.0f - d.NdotV, 5.0f));
+    float FDL = 1.0f + (FD90MinusOne * pow5(1.0f - d.NdotL));
+    float FDV = 1.0f + (FD90MinusOne * pow5(1.0f - d.NdotV));
     return FDL * FDV * energyFactor;
 }
 GB_D BrdfData prepare_brdf(float3 N, float3 L, float3 V, const MatBrdf& m) {  // prepareBRDFData, :527-564
@@ -360,15 +369,32 @@ GB_D float3 offset_ray(float3 p, float3 n) {
 // decoded per texel through a 256-entry table computed on the host).
 // Arithmetic is unfused so the any-hit alpha test matches the CPU exactly.
 // ---------------------------------------------------------------------------
-static __constant__ float c_srgb_lut[256];  // filled per translation unit by its init function
+// 8-bit channel values as floats: entries 0..255 sRGB-decoded, 256..511 c / 255
+// (IEEE).  Filled per translation unit by its init function.  In global
+// memory, not constant memory: the lanes of a warp look up different values,
+// which the constant cache serves one after the other.
+static __device__ float g_texel_lut[512];
 
-GB_D int wrap_idx(int i, int n, uint32_t mode) {
-    if (mode == GBRT_WRAP_CLAMP_TO_EDGE) return min(max(i, 0), n - 1);
-    if (mode == GBRT_WRAP_MIRRORED_REPEAT) {
-        int m = ((i % (2 * n)) + 2 * n) % (2 * n);
-        return m < n ? m : 2 * n - 1 - m;
+// Both neighbours i, i + 1 on an axis of n texels.
+GB_D int2 wrap_pair(int i, int n, uint32_t mode) {
+    if (mode == GBRT_WRAP_CLAMP_TO_EDGE) {
+        const int j = (int)((uint32_t)i + 1u);
+        return make_int2(min(max(i, 0), n - 1), min(max(j, 0), n - 1));
     }
-    return ((i % n) + n) % n;
+    // the remainder of i, and of i + 1 from it (i + 1 past the largest int starts over)
+    const int period = mode == GBRT_WRAP_MIRRORED_REPEAT ? 2 * n : n;
+    auto rem = [&](int v) {
+        if (!(period & (period - 1))) return v & (period - 1);
+        const int m = v % period;
+        return m < 0 ? m + period : m;
+    };
+    int a = rem(i);
+    int b = i == 0x7FFFFFFF ? rem((int)0x80000000u) : (a + 1 == period ? 0 : a + 1);
+    if (mode == GBRT_WRAP_MIRRORED_REPEAT) {
+        a = a < n ? a : period - 1 - a;
+        b = b < n ? b : period - 1 - b;
+    }
+    return make_int2(a, b);
 }
 GB_D float half_bits_to_float(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 GB_D float4 tex_fetch(const DevTexture& t, int x, int y) {
@@ -380,10 +406,8 @@ GB_D float4 tex_fetch(const DevTexture& t, int x, int y) {
                   half_bits_to_float(raw.y & 0xFFFF), half_bits_to_float(raw.y >> 16));
     }
     uchar4 p = __ldg(reinterpret_cast<const uchar4*>(t.data) + k);
-    if (t.format == GBRT_TEX_RGBA8_SRGB)
-        return f4(c_srgb_lut[p.x], c_srgb_lut[p.y], c_srgb_lut[p.z], __fdiv_rn((float)p.w, 255.0f));
-    return f4(__fdiv_rn((float)p.x, 255.0f), __fdiv_rn((float)p.y, 255.0f), __fdiv_rn((float)p.z, 255.0f),
-              __fdiv_rn((float)p.w, 255.0f));
+    const float* rgb = g_texel_lut + (t.format == GBRT_TEX_RGBA8_SRGB ? 0 : 256);
+    return f4(__ldg(rgb + p.x), __ldg(rgb + p.y), __ldg(rgb + p.z), __ldg(g_texel_lut + 256 + p.w));
 }
 GB_D float lerp_rn(float a, float b, float f) { return add_rn(mul_rn(a, sub_rn(1.0f, f)), mul_rn(b, f)); }
 GB_D float4 lerp4_rn(float4 a, float4 b, float f) {
@@ -395,15 +419,34 @@ GB_D float4 sample_tex2d(const DevTexture& t, float u, float v) {
     float fx = floorf(x), fy = floorf(y);
     float ax = sub_rn(x, fx), ay = sub_rn(y, fy);
     int i0 = (int)fx, j0 = (int)fy;
-    int xa = wrap_idx(i0, t.w, t.wrap_s), xb = wrap_idx(i0 + 1, t.w, t.wrap_s);
-    int ya = wrap_idx(j0, t.h, t.wrap_t), yb = wrap_idx(j0 + 1, t.h, t.wrap_t);
-    float4 top = lerp4_rn(tex_fetch(t, xa, ya), tex_fetch(t, xb, ya), ax);
-    float4 bot = lerp4_rn(tex_fetch(t, xa, yb), tex_fetch(t, xb, yb), ax);
+    const int2 xs = wrap_pair(i0, (int)t.w, t.wrap_s), ys = wrap_pair(j0, (int)t.h, t.wrap_t);
+    float4 top = lerp4_rn(tex_fetch(t, xs.x, ys.x), tex_fetch(t, xs.y, ys.x), ax);
+    float4 bot = lerp4_rn(tex_fetch(t, xs.x, ys.y), tex_fetch(t, xs.y, ys.y), ax);
     return lerp4_rn(top, bot, ay);
+}
+// Shading's texture samples, out of line: closest_hit takes up to a dozen, and
+// inlined they made it so large that its warps waited for instructions two
+// thirds of the time.
+static __device__ __noinline__ float4 sample_tex2d_call(const void* data, uint32_t w, uint32_t h, uint32_t format,
+                                                        uint32_t wrap_s, uint32_t wrap_t, float u, float v) {
+    DevTexture t;
+    t.data = data;
+    t.w = w;
+    t.h = h;
+    t.format = format;
+    t.wrap_s = wrap_s;
+    t.wrap_t = wrap_t;
+    return sample_tex2d(t, u, v);
 }
 GB_D float4 texture(const DevScene& s, int idx, float2 uv) {
     if (idx < 0 || (uint32_t)idx >= s.ntex || s.tex[idx].w == 0) return f4(1.0f, 1.0f, 1.0f, 1.0f);
-    return sample_tex2d(s.tex[idx], uv.x, uv.y);
+    const DevTexture& t = s.tex[idx];
+    return sample_tex2d_call(t.data, t.w, t.h, t.format, t.wrap_s, t.wrap_t, uv.x, uv.y);
+}
+// The alpha channel alone, in line, for the any-hit test.
+GB_D float texture_alpha(const DevScene& s, int idx, float2 uv) {
+    if (idx < 0 || (uint32_t)idx >= s.ntex || s.tex[idx].w == 0) return 1.0f;
+    return sample_tex2d(s.tex[idx], uv.x, uv.y).w;
 }
 GB_D float2 get_uv(float4 uv01, int index) {  // getUV, Commons.glsl:65-72
     if (index == 0) return make_float2(uv01.x, uv01.y);
@@ -432,7 +475,8 @@ GB_D float3 sample_sky(const DevScene& s, float3 d) {
     t.w = t.h = s.sky_size;
     t.format = s.sky_format;
     t.wrap_s = t.wrap_t = GBRT_WRAP_CLAMP_TO_EDGE;
-    float4 r = sample_tex2d(t, 0.5f * (sc / ma + 1.0f), 0.5f * (tc / ma + 1.0f));
+    float4 r = sample_tex2d_call(t.data, t.w, t.h, t.format, t.wrap_s, t.wrap_t, 0.5f * (sc / ma + 1.0f),
+                                 0.5f * (tc / ma + 1.0f));
     return f3(r.x, r.y, r.z);
 }
 

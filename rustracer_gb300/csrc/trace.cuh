@@ -147,12 +147,12 @@ GB_D bool anyhit_ignore(const DevScene& s, uint32_t custom, uint32_t prim, uint3
     if (mat.workflow == 1u) {  // SPECULAR_GLOSS_WORKFLOW
         float da = mat.sg_diffuse_factor[3];
         if (mat.sg_diffuse_texture.index >= 0)
-            da = mul_rn(da, texture(s, mat.sg_diffuse_texture.index, uvset(mat.sg_diffuse_texture.coord)).w);
+            da = mul_rn(da, texture_alpha(s, mat.sg_diffuse_texture.index, uvset(mat.sg_diffuse_texture.coord)));
         opacity = mul_rn(ca, da);
     } else {
         opacity = mul_rn(ca, mat.base_color[3]);
         if (mat.base_color_texture.index >= 0)
-            opacity = mul_rn(opacity, texture(s, mat.base_color_texture.index, uvset(mat.base_color_texture.coord)).w);
+            opacity = mul_rn(opacity, texture_alpha(s, mat.base_color_texture.index, uvset(mat.base_color_texture.coord)));
     }
     if (alpha_mode == 2u) return opacity < mat.alpha_cutoff;  // MASK
     const float uu = u2f(pcg4d(make_uint4(c.px, c.py, c.sample, blend_hash(inst, prim, c.tag))).x);

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <cstring>
 
+#define GBRT_FULL_SHADE
 #include "wavefront.cuh"
 
 namespace gbrt {
@@ -78,8 +79,8 @@ __global__ void __launch_bounds__(128) wfm_finish(WfState st) {
 }
 
 // --- host side ---------------------------------------------------------------
-cudaError_t init_wave_multi_constants(const float* srgb_lut) {
-    return cudaMemcpyToSymbol(c_srgb_lut, srgb_lut, 256 * sizeof(float));
+cudaError_t init_wave_multi_constants(const float* texel_lut) {
+    return cudaMemcpyToSymbol(g_texel_lut, texel_lut, 512 * sizeof(float));
 }
 
 namespace {

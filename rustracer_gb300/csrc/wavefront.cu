@@ -6,7 +6,7 @@
 // segment -- travels as a __grid_constant__ kernel parameter, so the scene
 // pointers the traversal reads every step are constant-bank operands.  The
 // kernel bodies are in wavefront.cuh; the batched form is wave_multi.cu.
-#include "wavefront.cuh"
+#include "single_wave.cuh"
 
 namespace gbrt_host {
 cudaError_t nrc_query_counted(gbrt_nrc* r, const float4* q, const uint32_t* n_dev, uint32_t n_max, float4* out,
@@ -14,25 +14,6 @@ cudaError_t nrc_query_counted(gbrt_nrc* r, const float4* q, const uint32_t* n_de
 }
 
 namespace gbrt {
-
-namespace {
-
-// One job and one segment; every block serves it.
-struct SingleWave {
-    WaveJob J;
-    WaveSeg S;
-    GB_D uint32_t block_job(int) const { return 0; }
-    GB_D uint32_t blk0(int, uint32_t) const { return 0; }
-    GB_D uint32_t nblk(int, uint32_t) const { return gridDim.x; }
-    GB_D const WaveJob& job(uint32_t) const { return J; }
-    GB_D const WaveSeg& seg(uint32_t) const { return S; }
-    GB_D uint32_t seg_of_path(uint32_t) const { return 0; }
-    GB_D uint32_t seg_of_fin(uint32_t) const { return 0; }
-    GB_D uint32_t npaths() const { return S.k * S.npw; }
-    GB_D uint32_t nfin() const { return S.npw; }
-};
-
-}  // namespace
 
 __global__ void __launch_bounds__(128) wf_camera(const __grid_constant__ SingleWave w, WfState st) {
     camera_body(w, st, blockIdx.x * blockDim.x + threadIdx.x);
@@ -42,14 +23,12 @@ __global__ void __launch_bounds__(128, trace_minb(kMode))
     wf_extend(const __grid_constant__ SingleWave w, WfState st, uint32_t b) {
     extend_body<kMode>(w, st, b, 0u);
 }
-// kFeat: the material features compiled in (kFeatAll, or 0 for scenes
-// without textures, specular-glossiness or debug shading, whose smaller body
-// runs at more resident blocks).
-template <uint32_t kFeat>
-__global__ void __launch_bounds__(kFeat ? kShadeThreads : kShadePlainThreads,
-                                  kFeat ? kShadeMinBlocks : kShadePlainMinBlocks)
-    wf_shade(const __grid_constant__ SingleWave w, WfState st, uint32_t b) {
-    shade_body<SingleWave, false, kFeat>(w, st, b);
+// The form for scenes without textures, specular-glossiness, volumes or debug
+// shading, whose smaller body runs at more resident blocks (the others:
+// shade_full.cu).
+__global__ void __launch_bounds__(kShadePlainThreads, kShadePlainMinBlocks)
+    wf_shade_plain(const __grid_constant__ SingleWave w, WfState st, uint32_t b) {
+    shade_body<SingleWave, false, 0u>(w, st, b);
 }
 template <int kMode>
 __global__ void __launch_bounds__(128, trace_minb(kMode))
@@ -60,12 +39,8 @@ __global__ void __launch_bounds__(128) wf_finish(const __grid_constant__ SingleW
     finish_body(w, st, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// Radiance-cache forms of shade and finish, and the step that adds
-// throughput x cache output to the paths that stopped at bounce b.
-__global__ void __launch_bounds__(kShadeThreads, kShadeMinBlocks) wf_shade_nrc(const __grid_constant__ SingleWave w, WfState st, uint32_t b,
-                                                    const __grid_constant__ NrcWave nrc) {
-    shade_body<SingleWave, true>(w, st, b, &nrc);
-}
+// Radiance-cache form of finish, and the step that adds throughput x cache
+// output to the paths that stopped at bounce b.
 __global__ void __launch_bounds__(128) wf_finish_nrc(const __grid_constant__ SingleWave w, WfState st,
                                                      const __grid_constant__ NrcWave nrc) {
     finish_body<SingleWave, true>(w, st, blockIdx.x * blockDim.x + threadIdx.x, &nrc);
@@ -97,8 +72,8 @@ __global__ void __launch_bounds__(128) wf_resolve(gbrt_ubo ubo, RenderOut out, c
 }
 
 // --- host side ---------------------------------------------------------------
-cudaError_t init_wavefront_constants(const float* srgb_lut) {
-    return cudaMemcpyToSymbol(c_srgb_lut, srgb_lut, 256 * sizeof(float));
+cudaError_t init_wavefront_constants(const float* texel_lut) {
+    return cudaMemcpyToSymbol(g_texel_lut, texel_lut, 512 * sizeof(float));
 }
 
 namespace {
@@ -116,10 +91,10 @@ cudaError_t grids(Grid& g) {
     int sms = 0, be = 0, bs = 0, bh = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&be, wf_extend<kTraceWide>, 128, 0)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bs, wf_shade<kFeatAll>, kShadeThreads, 0)) != cudaSuccess)
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bs, shade_full_kernel(false), kShadeThreads, 0)) != cudaSuccess)
         return e;
     int bp = 0;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bp, wf_shade<0u>, kShadePlainThreads, 0)) != cudaSuccess)
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bp, wf_shade_plain, kShadePlainThreads, 0)) != cudaSuccess)
         return e;
     g.shade_plain = sms * (bp > 0 ? bp : 1);
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bh, wf_shadow<kTraceWide>, 128, 0)) != cudaSuccess) return e;
@@ -261,9 +236,8 @@ cudaError_t launch_wavefront(const DevScene& s, const gbrt_ubo& ubo, const Rende
                 te();
                 if (side && b > 0 && (e = cudaStreamWaitEvent(stream, side->shadowed, 0)) != cudaSuccess) return e;
                 tb(1);
-                if (nrc) wf_shade_nrc<<<bs, ts, 0, stream>>>(w, st, b, *nrc);
-                else if (feat == 0u) wf_shade<0u><<<bp, tp, 0, stream>>>(w, st, b);
-                else wf_shade<kFeatAll><<<bs, ts, 0, stream>>>(w, st, b);
+                if (nrc || feat) launch_shade_full(w, st, b, nrc, bs, ts, stream);
+                else wf_shade_plain<<<bp, tp, 0, stream>>>(w, st, b);
                 te();
                 if (nrc && !nrc->disabled && (nrc->mode == 1u ? b == 0 : b >= 1)) {  // queries of the paths that stopped here
                     tb(3);
