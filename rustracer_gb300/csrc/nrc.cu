@@ -111,6 +111,56 @@ GB_D void nrc_encode_h(const NrcView& v, float3 p, float (&x)[kNrcIn]) {
     }
 }
 
+// Table reads of a query: levels that fit the first-level cache (the coarsest
+// three: 23, 63 and 171 KB at base 16 and growth 1.447) go through it, the
+// others, which never hit there, straight to the second.
+constexpr int kCachedLevels = 3;
+GB_D uint4 table_quad(const __half2* grid, uint32_t i, bool cached) {  // entries 4 i .. 4 i + 3
+    const uint4* p = reinterpret_cast<const uint4*>(grid) + i;
+    return cached ? __ldg(p) : __ldcg(p);
+}
+GB_D uint32_t table_entry(const __half2* grid, uint32_t i, bool cached) {
+    const uint32_t* p = reinterpret_cast<const uint32_t*>(grid) + i;
+    return cached ? __ldg(p) : __ldcg(p);
+}
+
+// FP16 encoding of every other pair of levels of one point, from pair `half`
+// on (16 features).  The corners at x and x + 1 have neighbouring entries
+// unless x ends in binary 11 (dense levels: unless the index does), so one
+// 16-byte read usually serves both: the queries are bound by the number of
+// reads that go to the second-level cache.
+GB_D void nrc_encode_h8(const NrcView& v, float3 p, int half, float (&x)[16]) {
+#pragma unroll
+    for (int l = 0; l < 8; ++l) {
+        const int level = (l & 1) + 4 * (l >> 1) + 2 * half;
+        const bool cached = level < kCachedLevels;
+        uint32_t idx[8], e[8];
+        float w[8];
+#pragma unroll
+        for (int c = 0; c < 8; ++c) nrc_corner(v, level, p, c, idx[c], w[c]);
+#pragma unroll
+        for (int c = 0; c < 8; c += 2) {
+            const uint4 g = table_quad(v.grid_h, idx[c] >> 2, cached);
+            auto pick = [&](uint32_t i) {
+                const uint32_t a = i & 1u ? g.y : g.x, b = i & 1u ? g.w : g.z;
+                return i & 2u ? b : a;
+            };
+            e[c] = pick(idx[c]);
+            e[c + 1] = pick(idx[c + 1]);
+            if ((idx[c] ^ idx[c + 1]) >> 2) e[c + 1] = table_entry(v.grid_h, idx[c + 1], cached);
+        }
+        float f0 = 0.0f, f1 = 0.0f;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            const float2 t = __half22float2(*reinterpret_cast<const __half2*>(&e[c]));
+            f0 = fmaf(w[c], t.x, f0);
+            f1 = fmaf(w[c], t.y, f1);
+        }
+        x[2 * l] = f0;
+        x[2 * l + 1] = f1;
+    }
+}
+
 constexpr int kInferWarps = 4;
 constexpr int kInRow = kNrcIn + kPadK;  // 40 BF16 per input row
 constexpr size_t kInferSmem = (size_t)kBf16Padded * 2 + (size_t)kInferWarps * 32 * kInRow * 2;
@@ -186,9 +236,9 @@ __global__ void __launch_bounds__(128) nrc_infer_kernel(NrcView v, const float4*
 }
 
 // ---------------------------------------------------------------------------
-// Queries on the 5th-generation tensor cores (tcgen05).  A CTA of 128 threads
-// takes 128 queries per step: thread i encodes query i into row i of the A
-// tile (shared memory, BF16, K-major canonical layout without swizzle: 8x8
+// Queries on the 5th-generation tensor cores (tcgen05).  A CTA of 256 threads
+// takes 128 queries per step: threads i and i + 128 encode query i into row i of
+// the A tile (shared memory, BF16, K-major canonical layout without swizzle: 8x8
 // core matrices of 128 B, K-adjacent ones 128 B apart, 8-row groups K*16 B
 // apart); one elected thread issues the layer's tcgen05.mma (M = 128, N = 64
 // or 16, K = 16 per instruction) with the FP32 accumulator in tensor memory
@@ -199,12 +249,19 @@ __global__ void __launch_bounds__(128) nrc_infer_kernel(NrcView v, const float4*
 // *status and stops issuing work.
 
 constexpr uint32_t kTcTimeout = 1u;
+// CTAs per SM.  Four fill the shared memory and leave the first-level cache too
+// small to hold the table reads in flight: one million queries at 2 / 3 / 4 CTAs
+// take 353 / 321 / 510 us (from one 4-byte read per corner, 128 threads and 4
+// CTAs: 629).
+constexpr int kTcBlocks = 3;
 constexpr int kTcRows = 128;
-// BF16 weights in core-matrix layout: layer l occupies out_l x in_l (W5 padded to 16 rows)
+constexpr int kTcThreads = 2 * kTcRows;  // thread t: row t % 128, half of its levels and of its columns
+// BF16 weights in core-matrix layout: layer l occupies out_l x in_l (W5 padded to 8 rows; the last layer's MMA
+// is 16 columns wide, the upper 8 of them, never read, multiply what follows in shared memory)
 __host__ __device__ constexpr int tc_w_off(int l) {  // in elements
     return l == 0 ? 0 : kNrcHidden * kNrcIn + (l - 1) * kNrcHidden * kNrcHidden;
 }
-constexpr int kTcWElems = tc_w_off(5) + 16 * kNrcHidden;                    // 19,456
+constexpr int kTcWElems = tc_w_off(5) + 8 * kNrcHidden;                     // 18,944
 constexpr size_t kTcSmem = (size_t)kTcWElems * 2 + (size_t)kTcRows * kNrcHidden * 2 + 64;
 
 // byte offset of element (row, k) in a K-major no-swizzle tile with K columns
@@ -255,7 +312,7 @@ GB_D bool tc_wait(uint32_t mbar, uint32_t phase) {
                    "=r"(v[14]), "=r"(v[15])                                                                     \
                  : "r"(base))
 
-__global__ void __launch_bounds__(128, 1) nrc_infer_tc_kernel(NrcView v, const float4* __restrict__ q, uint32_t n,
+__global__ void __launch_bounds__(kTcThreads, kTcBlocks) nrc_infer_tc_kernel(NrcView v, const float4* __restrict__ q, uint32_t n,
                                                               float4* __restrict__ out, const uint32_t* n_dev,
                                                               const __nv_bfloat16* __restrict__ wtc,
                                                               uint32_t* status) {
@@ -288,24 +345,21 @@ __global__ void __launch_bounds__(128, 1) nrc_infer_tc_kernel(NrcView v, const f
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     const uint32_t tmem = *tslot;
-    const uint32_t tlane = tmem + ((warp * 32u) << 16);  // this warp's 32 lanes
+    const uint32_t row = tid & (kTcRows - 1u), half = tid / kTcRows;
+    const uint32_t tlane = tmem + (((warp & 3u) * 32u) << 16);  // this warp's 32 lanes
     uint32_t phase = 0;
     bool ok = true;
     for (uint32_t base = blockIdx.x * kTcRows; base < n && ok; base += gridDim.x * kTcRows) {
-        const uint32_t i = base + tid;
+        const uint32_t i = base + row;
         {
-            float x[kNrcIn];
             const float4 qi = i < n ? q[i] : f4(0.0f, 0.0f, 0.0f, 0.0f);
-            nrc_encode_h(v, nrc_normalise(v, f3(qi)), x);
+            const float3 pn = nrc_normalise(v, f3(qi));
+            float x[kNrcIn / 2];
+            nrc_encode_h8(v, pn, (int)half, x);
 #pragma unroll
-            for (int k = 0; k < kNrcIn; k += 8) {
-                uint4 pk;
-                pk.x = pack_bf16(x[k], x[k + 1]);
-                pk.y = pack_bf16(x[k + 2], x[k + 3]);
-                pk.z = pack_bf16(x[k + 4], x[k + 5]);
-                pk.w = pack_bf16(x[k + 6], x[k + 7]);
-                *reinterpret_cast<uint4*>(sa + tc_core_off(tid, k, kNrcIn)) = pk;
-            }
+            for (int k = 0; k < kNrcIn / 2; k += 4)  // two levels: four features from column 2 k + 4 half on
+                *reinterpret_cast<uint2*>(sa + tc_core_off(row, 2 * k + 4 * half, kNrcIn)) =
+                    make_uint2(pack_bf16(x[k], x[k + 1]), pack_bf16(x[k + 2], x[k + 3]));
         }
         float y[3] = {0.0f, 0.0f, 0.0f};
         for (int l = 0; l < 6 && ok; ++l) {
@@ -331,9 +385,10 @@ __global__ void __launch_bounds__(128, 1) nrc_infer_tc_kernel(NrcView v, const f
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             if (l < 5) {
 #pragma unroll
-                for (int c = 0; c < kNrcHidden; c += 16) {
+                for (int j = 0; j < kNrcHidden / 2; j += 16) {
+                    const uint32_t c = half * (kNrcHidden / 2) + j;
                     uint32_t r[16];
-                    TC_LD16(tlane + (uint32_t)c, r);
+                    TC_LD16(tlane + c, r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 #pragma unroll
                     for (int k = 0; k < 16; k += 8) {
@@ -342,10 +397,10 @@ __global__ void __launch_bounds__(128, 1) nrc_infer_tc_kernel(NrcView v, const f
                         pk.y = pack_bf16(fmaxf(__uint_as_float(r[k + 2]), 0.0f), fmaxf(__uint_as_float(r[k + 3]), 0.0f));
                         pk.z = pack_bf16(fmaxf(__uint_as_float(r[k + 4]), 0.0f), fmaxf(__uint_as_float(r[k + 5]), 0.0f));
                         pk.w = pack_bf16(fmaxf(__uint_as_float(r[k + 6]), 0.0f), fmaxf(__uint_as_float(r[k + 7]), 0.0f));
-                        *reinterpret_cast<uint4*>(sa + tc_core_off(tid, c + k, kNrcHidden)) = pk;
+                        *reinterpret_cast<uint4*>(sa + tc_core_off(row, c + k, kNrcHidden)) = pk;
                     }
                 }
-            } else {
+            } else if (half == 0) {  // uniform in the warp
                 uint32_t r[16];
                 TC_LD16(tlane, r);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
@@ -354,7 +409,7 @@ __global__ void __launch_bounds__(128, 1) nrc_infer_tc_kernel(NrcView v, const f
                 y[2] = __uint_as_float(r[2]);
             }
         }
-        if (ok && i < n) out[i] = f4(y[0], y[1], y[2], q[i].w);
+        if (ok && half == 0 && i < n) out[i] = f4(y[0], y[1], y[2], q[i].w);
     }
     if (!ok) {
         if (status && tid == 0) atomicOr(status, kTcTimeout);
@@ -366,7 +421,7 @@ __global__ void __launch_bounds__(128, 1) nrc_infer_tc_kernel(NrcView v, const f
 }
 
 // FP32 masters -> BF16 weights in the core-matrix order of the tcgen05
-// kernel (W5 padded to 16 rows with zeros).
+// kernel (W5 padded to 8 rows with zeros).
 __global__ void nrc_tc_weights_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ wtc) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= kTcWElems) return;
@@ -1058,16 +1113,16 @@ cudaError_t nrc_kernel_setup(gbrt_nrc* r) {
         r->train_blocks = sms * std::max(per_train, 1);
         e = cudaFuncSetAttribute(nrc_infer_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcSmem);
         if (e != cudaSuccess) return e;
-        cudaFuncSetAttribute(nrc_infer_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                             (int)cudaSharedmemCarveoutMaxShared);
+        // no more shared memory than the CTAs use: the rest holds the table reads in flight
+        cudaFuncSetAttribute(nrc_infer_tc_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 72);
         // CTAs per SM by shared memory (the occupancy query has reported 1 for this
-        // kernel where the launch fits 4), at most 4 x 64 tensor-memory columns
+        // kernel where the launch fits 4), at most kTcBlocks
         int smem_sm = 0, smem_rsv = 0, per_tc = 0;
         cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
         cudaDeviceGetAttribute(&smem_rsv, cudaDevAttrReservedSharedMemoryPerBlock, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_tc, nrc_infer_tc_kernel, 128, kTcSmem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_tc, nrc_infer_tc_kernel, kTcThreads, kTcSmem);
         per_tc = std::max(per_tc, smem_sm / (int)(kTcSmem + (size_t)smem_rsv));
-        r->tc_blocks = sms * std::max(std::min(per_tc, 4), 1);
+        r->tc_blocks = sms * std::max(std::min(per_tc, kTcBlocks), 1);
     }
     return cudaSuccess;
 }
@@ -1079,7 +1134,7 @@ cudaError_t nrc_query_device(gbrt_nrc* r, const float4* q, uint32_t n, float4* o
     if (e != cudaSuccess) return e;
     if (!(r->cfg.flags & GBRT_NRC_QUERY_MMA_SYNC)) {
         const uint32_t need = (n + kTcRows - 1) / kTcRows;
-        nrc_infer_tc_kernel<<<std::min<uint32_t>(need, (uint32_t)r->tc_blocks), 128, kTcSmem, st>>>(
+        nrc_infer_tc_kernel<<<std::min<uint32_t>(need, (uint32_t)r->tc_blocks), kTcThreads, kTcSmem, st>>>(
             r->view, q, n, out, nullptr, r->mlp_tc.as<__nv_bfloat16>(), r->status.as<uint32_t>());
         return cudaGetLastError();
     }
@@ -1094,7 +1149,7 @@ cudaError_t nrc_query_counted(gbrt_nrc* r, const float4* q, const uint32_t* n_de
     cudaError_t e = nrc_kernel_setup(r);
     if (e != cudaSuccess) return e;
     if (!(r->cfg.flags & GBRT_NRC_QUERY_MMA_SYNC))
-        nrc_infer_tc_kernel<<<r->tc_blocks, 128, kTcSmem, st>>>(r->view, q, n_max, out, n_dev,
+        nrc_infer_tc_kernel<<<r->tc_blocks, kTcThreads, kTcSmem, st>>>(r->view, q, n_max, out, n_dev,
                                                                 r->mlp_tc.as<__nv_bfloat16>(),
                                                                 r->status.as<uint32_t>());
     else
