@@ -53,6 +53,7 @@ constexpr uint32_t kWaveCapLarge = kMaxWavePaths < (1u << 26) ? kMaxWavePaths : 
 constexpr uint64_t kSoloPaths = 1ull << 24;
 constexpr uint32_t kChunkDiv = 8;             // pixel chunk = wave / 8 (finer packing)
 constexpr int kMaxInFlight = 2;
+constexpr uint64_t kPoolKeep = 256ull << 20;
 
 // Stream-ordered device buffer: cudaFree would wait for the whole device,
 // stalling the waves in flight.
@@ -60,9 +61,9 @@ struct AsyncBuf {
     void* p = nullptr;
     size_t bytes = 0;
     cudaStream_t st = nullptr;
-    cudaError_t alloc(size_t n, cudaStream_t s) {
+    cudaError_t alloc(size_t n, cudaMemPool_t pool, cudaStream_t s) {
         st = s;
-        cudaError_t e = cudaMallocAsync(&p, n, s);
+        cudaError_t e = cudaMallocFromPoolAsync(&p, n, pool, s);
         if (e == cudaSuccess) bytes = n;
         else p = nullptr;
         return e;
@@ -128,6 +129,9 @@ struct JobQueue {
     bool stop = false;
     std::thread worker;
     cudaStream_t dl = nullptr;  // downloads of finished jobs (non-blocking stream)
+    // the jobs' buffers: a pool that keeps up to kPoolKeep bytes between jobs
+    // (the default pool gives everything back at each wait)
+    cudaMemPool_t pool = nullptr;
 
     void run();
     bool admit_one(std::unique_lock<std::mutex>& lk);
@@ -194,9 +198,9 @@ bool JobQueue::admit_one(std::unique_lock<std::mutex>& lk) {
     while (inject && !ctx->inject_admit_oom.compare_exchange_weak(inject, inject - 1)) {
     }
     if (inject) e = cudaErrorMemoryAllocation;  // injected (host side): as if the allocation had failed
-    if (e == cudaSuccess) e = j->frame_sum.alloc((size_t)j->npix * sizeof(float4), st);
-    if (e == cudaSuccess && j->out_rgba8) e = j->img.alloc((size_t)j->npix * 4, st);
-    if (e == cudaSuccess) e = j->counters.alloc(sizeof(DeviceCounters), st);
+    if (e == cudaSuccess) e = j->frame_sum.alloc((size_t)j->npix * sizeof(float4), pool, st);
+    if (e == cudaSuccess && j->out_rgba8) e = j->img.alloc((size_t)j->npix * 4, pool, st);
+    if (e == cudaSuccess) e = j->counters.alloc(sizeof(DeviceCounters), pool, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(j->frame_sum.p, 0, j->frame_sum.bytes, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(j->counters.p, 0, sizeof(DeviceCounters), st);
     if (e != cudaSuccess) {
@@ -509,7 +513,13 @@ void jobs_shutdown(gbrt_ctx* c) {
         for (cudaEvent_t ev : q->free_events) cudaEventDestroy(ev);
         if (q->dl) cudaStreamDestroy(q->dl);
     }
-    delete q;
+    cudaMemPool_t pool = q->pool;
+    delete q;  // its jobs' buffers go back to the pool first
+    {
+        DeviceGuard g(c->device);
+        cudaStreamSynchronize(c->stream);
+        if (pool) cudaMemPoolDestroy(pool);
+    }
     c->jobs = nullptr;
 }
 
@@ -619,9 +629,19 @@ int gbrt_job_submit(gbrt_ctx* c, const gbrt_job_desc* d, uint64_t* job_id) {
             const uint64_t gib = 1ull << 30;
             q->budget = c->jobs_budget ? c->jobs_budget : (fr > gib ? fr - gib : fr / 2);
             if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&q->dl, cudaStreamNonBlocking);
+            if (e == cudaSuccess) {
+                cudaMemPoolProps props{};
+                props.allocType = cudaMemAllocationTypePinned;
+                props.location.type = cudaMemLocationTypeDevice;
+                props.location.id = c->device;
+                e = cudaMemPoolCreate(&q->pool, &props);
+                uint64_t keep = kPoolKeep;
+                if (e == cudaSuccess) e = cudaMemPoolSetAttribute(q->pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            }
             if (e == cudaSuccess) e = wavefront_reserve(c, q->deep_cap, 0) == cudaSuccess ? cudaSuccess : cudaErrorMemoryAllocation;
             if (e != cudaSuccess) {
                 if (q->dl) cudaStreamDestroy(q->dl);
+                if (q->pool) cudaMemPoolDestroy(q->pool);
                 return cuda_fail(c, e, "job scheduler setup");
             }
             c->jobs = q.release();

@@ -23,7 +23,7 @@ struct RenderOut {
 
 // wavefront.cu: device buffers of the wavefront path tracer, `cap` paths.
 // Each job of a wave owns kWfCounters queue lengths and fetch cursors.
-constexpr int kWfCounters = 128;
+constexpr int kWfCounters = 160;
 #ifndef GBRT_PID_BITS
 #define GBRT_PID_BITS 26
 #endif
@@ -98,13 +98,16 @@ struct WaveRing {
     cudaEvent_t ev[kSlots] = {};
     int next = 0;
     // captured launch sequences of batched waves, per traversal form (with
-    // or without kTraceOpaque) and bounce count, valid for the wavefront
-    // buffers in graph_state
-    cudaGraphExec_t graph[8][32] = {};
+    // or without kTraceOpaque), bounce count and shade kernels (1: plain, 2:
+    // full-feature, 3: both), valid for the wavefront buffers in graph_state
+    cudaGraphExec_t graph[8][32][4] = {};
     WfState graph_state{};
     // private stream the graphs are captured on: the launch stream is shared
     // with the API calls of other threads, which must not land in a capture
     cudaStream_t cap = nullptr;
+    // the shadow branch of a captured wave
+    cudaStream_t cap_side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
 };
 // Drops the captured graphs (the ring's buffers stay).
 void wave_graphs_reset(WaveRing& r);

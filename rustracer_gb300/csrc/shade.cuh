@@ -424,9 +424,11 @@ GB_D float4 sample_tex2d(const DevTexture& t, float u, float v) {
     float4 bot = lerp4_rn(tex_fetch(t, xs.x, ys.y), tex_fetch(t, xs.y, ys.y), ax);
     return lerp4_rn(top, bot, ay);
 }
-// Shading's texture samples, out of line: closest_hit takes up to a dozen, and
-// inlined they made it so large that its warps waited for instructions two
-// thirds of the time.
+// Texture samples of the full-feature shade kernels, out of line: closest_hit
+// takes up to a dozen, and inlined they made it so large that its warps waited
+// for instructions two thirds of the time (materials frame: shade 2.06 -> 1.42
+// ms).  The radiance-cache form keeps them in line, where its results are the
+// plain frame's to the bit.
 static __device__ __noinline__ float4 sample_tex2d_call(const void* data, uint32_t w, uint32_t h, uint32_t format,
                                                         uint32_t wrap_s, uint32_t wrap_t, float u, float v) {
     DevTexture t;
@@ -441,7 +443,11 @@ static __device__ __noinline__ float4 sample_tex2d_call(const void* data, uint32
 GB_D float4 texture(const DevScene& s, int idx, float2 uv) {
     if (idx < 0 || (uint32_t)idx >= s.ntex || s.tex[idx].w == 0) return f4(1.0f, 1.0f, 1.0f, 1.0f);
     const DevTexture& t = s.tex[idx];
+#ifndef GBRT_FULL_SHADE
+    return sample_tex2d(t, uv.x, uv.y);
+#else
     return sample_tex2d_call(t.data, t.w, t.h, t.format, t.wrap_s, t.wrap_t, uv.x, uv.y);
+#endif
 }
 // The alpha channel alone, in line, for the any-hit test.
 GB_D float texture_alpha(const DevScene& s, int idx, float2 uv) {

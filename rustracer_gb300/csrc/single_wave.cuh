@@ -20,10 +20,10 @@ struct SingleWave {
     GB_D uint32_t nfin() const { return S.npw; }
 };
 
-// shade_full.cu: the shade kernels with every material feature compiled in,
-// with or without a radiance cache, and (for occupancy queries) their symbols.
-void launch_shade_full(const SingleWave& w, const WfState& st, uint32_t b, const NrcWave* nrc, uint32_t blocks,
-                       uint32_t threads, cudaStream_t stream);
-const void* shade_full_kernel(bool nrc);
+// shade_full.cu: the shade kernel with every material feature compiled in, and
+// (for occupancy queries) its symbol.
+void launch_shade_full(const SingleWave& w, const WfState& st, uint32_t b, uint32_t blocks, uint32_t threads,
+                       cudaStream_t stream);
+const void* shade_full_kernel();
 
 }  // namespace gbrt

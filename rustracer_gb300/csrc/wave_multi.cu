@@ -67,7 +67,36 @@ __global__ void __launch_bounds__(128, trace_minb(kMode)) wfm_extend(WfState st,
     const uint32_t own = MultiWave{}.block_job(0), nj = c_wave.njobs;
     for (uint32_t t = 0; t < nj; ++t) extend_body<kMode>(MultiWave{}, st, b, own + t < nj ? own + t : own + t - nj);
 }
-__global__ void __launch_bounds__(kShadeThreads, kShadeMinBlocks) wfm_shade(WfState st, uint32_t b) { shade_body(MultiWave{}, st, b); }
+// Shading a path costs several times more in one scene than in another, so
+// blocks go on to the other jobs here as well; jobs whose scenes need no
+// textures, specular-glossiness, volumes or debug shading run in the smaller
+// kernel.  24 frames of 256 x 256 x 2 of three scenes: 7.30 -> 6.41 ms, with the
+// shadow branch of the captured graph and the pool of job buffers.
+template <uint32_t kFeat>
+__global__ void __launch_bounds__(kFeat ? kShadeThreads : kShadePlainThreads, kFeat ? kShadeMinBlocks : kShadePlainMinBlocks)
+    wfm_shade(WfState st, uint32_t b) {
+    __shared__ uint32_t s_chunk;
+    const uint32_t own = MultiWave{}.block_job(1), nj = c_wave.njobs;
+    for (uint32_t t = 0; t < nj; ++t) {
+        const uint32_t j = own + t < nj ? own + t : own + t - nj;
+        if ((job_features(c_wave.jobs[j].s, c_wave.jobs[j].ubo) != 0u) != (kFeat != 0u)) continue;
+        uint32_t* cnt = st.counts + j * kWfCounters;
+        const uint32_t n = cnt[kQueue + b];
+        PathStats ps{0, 0, 0, 0, 0};
+        for (;;) {  // the block's next chunk of the job's queue
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                uint32_t* cursor = &cnt[kWorkShade + b];
+                s_chunk = __ldcg(cursor) < n ? atomicAdd(cursor, blockDim.x) : n;
+            }
+            __syncthreads();
+            const uint32_t first = s_chunk;
+            if (first >= n) break;
+            shade_range<MultiWave, false, kFeat>(MultiWave{}, st, b, j, first, min(n, first + blockDim.x), blockDim.x, ps);
+        }
+        flush_shade_stats(ps, c_wave.jobs[j].out.counters);
+    }
+}
 template <int kMode>
 __global__ void __launch_bounds__(128, trace_minb(kMode)) wfm_shadow(WfState st, uint32_t b) {
     const uint32_t own = MultiWave{}.block_job(2), nj = c_wave.njobs;
@@ -86,7 +115,7 @@ cudaError_t init_wave_multi_constants(const float* texel_lut) {
 namespace {
 struct Grid {
     int dev = -1;
-    int extend = 0, shade = 0, shadow = 0;
+    int extend = 0, shade = 0, shade_plain = 0, shadow = 0;
 };
 Grid g_grid;
 
@@ -95,13 +124,17 @@ cudaError_t grids(Grid& g) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (g.dev == dev) return cudaSuccess;
-    int sms = 0, be = 0, bs = 0, bh = 0;
+    int sms = 0, be = 0, bs = 0, bp = 0, bh = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&be, wfm_extend<kTraceWide>, 128, 0)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bs, wfm_shade, kShadeThreads, 0)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bs, wfm_shade<kFeatAll>, kShadeThreads, 0)) != cudaSuccess)
+        return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bp, wfm_shade<0u>, kShadePlainThreads, 0)) != cudaSuccess)
+        return e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bh, wfm_shadow<kTraceWide>, 128, 0)) != cudaSuccess) return e;
     g.extend = sms * (be > 0 ? be : 1);
     g.shade = sms * (bs > 0 ? bs : 1);
+    g.shade_plain = sms * (bp > 0 ? bp : 1);
     g.shadow = sms * (bh > 0 ? bh : 1);
     g.dev = dev;
     return cudaSuccess;
@@ -121,8 +154,10 @@ cudaError_t wave_ring_init(WaveRing& r) {
             return e;
         }
     }
-    if ((e = cudaStreamCreateWithFlags(&r.cap, cudaStreamNonBlocking)) != cudaSuccess) {
-        r.cap = nullptr;
+    if ((e = cudaStreamCreateWithFlags(&r.cap, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaStreamCreateWithFlags(&r.cap_side, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&r.fork, cudaEventDisableTiming)) != cudaSuccess ||
+        (e = cudaEventCreateWithFlags(&r.join, cudaEventDisableTiming)) != cudaSuccess) {
         wave_ring_free(r);
         return e;
     }
@@ -142,7 +177,11 @@ void wave_ring_free(WaveRing& r) {
     if (r.host) cudaFreeHost(r.host);
     r.host = nullptr;
     if (r.cap) cudaStreamDestroy(r.cap);
-    r.cap = nullptr;
+    if (r.cap_side) cudaStreamDestroy(r.cap_side);
+    if (r.fork) cudaEventDestroy(r.fork);
+    if (r.join) cudaEventDestroy(r.join);
+    r.cap = r.cap_side = nullptr;
+    r.fork = r.join = nullptr;
 }
 
 cudaError_t wave_acquire(WaveRing& r, WaveDesc** slot) {
@@ -197,7 +236,10 @@ int wave_mode(const WaveDesc& w) {
 
 // The launches of one batched wave with `nb` bounces in traversal form
 // `mode`; every grid is fixed, the wave itself is read from c_wave.
-cudaError_t enqueue_wave(const WfState& st, int mode, uint32_t nb, cudaStream_t stream, StageTimer* timer) {
+// shading: 1 plain, 2 full-feature, 3 both.  With `ring` (a capture) the shadow
+// stage is a branch beside the next extension, as in single frames.
+cudaError_t enqueue_wave(const WfState& st, int mode, uint32_t nb, int shading, cudaStream_t stream, StageTimer* timer,
+                         const WaveRing* ring) {
     cudaError_t e = cudaMemsetAsync(st.counts, 0, (size_t)kMaxWaveJobs * kWfCounters * sizeof(uint32_t), stream);
     if (e != cudaSuccess) return e;
     auto tb = [&](int stage) {
@@ -217,13 +259,23 @@ cudaError_t enqueue_wave(const WfState& st, int mode, uint32_t nb, cudaStream_t 
         tb(0);
         GBRT_TRACE_LAUNCH(wfm_extend, g_grid.extend, 128, stream, st, b);
         te();
+        if (ring && b > 0 && (e = cudaStreamWaitEvent(stream, ring->join, 0)) != cudaSuccess) return e;
         tb(1);
-        wfm_shade<<<g_grid.shade, kShadeThreads, 0, stream>>>(st, b);
+        if (shading & 2) wfm_shade<kFeatAll><<<g_grid.shade, kShadeThreads, 0, stream>>>(st, b);
+        if (shading & 1) wfm_shade<0u><<<g_grid.shade_plain, kShadePlainThreads, 0, stream>>>(st, b);
         te();
         tb(2);
-        GBRT_TRACE_LAUNCH(wfm_shadow, g_grid.shadow, 128, stream, st, b);
+        cudaStream_t ss = stream;
+        if (ring) {
+            if ((e = cudaEventRecord(ring->fork, stream)) != cudaSuccess) return e;
+            if ((e = cudaStreamWaitEvent(ring->cap_side, ring->fork, 0)) != cudaSuccess) return e;
+            ss = ring->cap_side;
+        }
+        GBRT_TRACE_LAUNCH(wfm_shadow, g_grid.shadow, 128, ss, st, b);
+        if (ring && (e = cudaEventRecord(ring->join, ss)) != cudaSuccess) return e;
         te();
     }
+    if (ring && nb && (e = cudaStreamWaitEvent(stream, ring->join, 0)) != cudaSuccess) return e;
     tb(3);
     wfm_finish<<<flat, 128, 0, stream>>>(st);
     te();
@@ -233,12 +285,13 @@ cudaError_t enqueue_wave(const WfState& st, int mode, uint32_t nb, cudaStream_t 
 }  // namespace
 
 void wave_graphs_reset(WaveRing& r) {
-    for (auto& row : r.graph)
-        for (auto& g : row)
-            if (g) {
-                cudaGraphExecDestroy(g);
-                g = nullptr;
-            }
+    for (auto& form : r.graph)
+        for (auto& row : form)
+            for (auto& g : row)
+                if (g) {
+                    cudaGraphExecDestroy(g);
+                    g = nullptr;
+                }
     r.graph_state = WfState{};
 }
 
@@ -255,21 +308,23 @@ cudaError_t launch_wave(WaveRing& ring, const WfState& st, cudaStream_t stream, 
     if ((e = cudaEventRecord(ring.ev[ring.next], stream)) != cudaSuccess) return e;
     ring.next = (ring.next + 1) % WaveRing::kSlots;
     const int mode = wave_mode(w);
+    int shading = 0;
+    for (uint32_t j = 0; j < w.njobs; ++j) shading |= job_features(w.jobs[j].s, w.jobs[j].ubo) ? 2 : 1;
     if (timer) {
         if ((e = stage_timer_reserve(*timer, timer->used + 2 + 3 * (int)w.nb + 1)) != cudaSuccess) return e;
-        return enqueue_wave(st, mode, w.nb, stream, timer);
+        return enqueue_wave(st, mode, w.nb, shading, stream, timer, nullptr);
     }
-    // one CUDA graph per (traversal form, bounce count), captured on first use
+    // one CUDA graph per (traversal form, bounce count, shade kernels), captured on first use
     // and replayed for every later wave; rebuilt when the wavefront buffers move
     if (std::memcmp(&ring.graph_state, &st, sizeof(WfState)) != 0) {
         wave_graphs_reset(ring);
         ring.graph_state = st;
     }
-    cudaGraphExec_t& exec = ring.graph[mode][w.nb];
+    cudaGraphExec_t& exec = ring.graph[mode][w.nb][shading];
     if (!exec) {
         cudaGraph_t graph = nullptr;
         if ((e = cudaStreamBeginCapture(ring.cap, cudaStreamCaptureModeThreadLocal)) != cudaSuccess) return e;
-        const cudaError_t ee = enqueue_wave(st, mode, w.nb, ring.cap, nullptr);
+        const cudaError_t ee = enqueue_wave(st, mode, w.nb, shading, ring.cap, nullptr, &ring);
         e = cudaStreamEndCapture(ring.cap, &graph);
         if (ee != cudaSuccess) e = ee;
         if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);

@@ -39,8 +39,12 @@ __global__ void __launch_bounds__(128) wf_finish(const __grid_constant__ SingleW
     finish_body(w, st, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// Radiance-cache form of finish, and the step that adds throughput x cache
-// output to the paths that stopped at bounce b.
+// Radiance-cache forms of shade and finish, and the step that adds throughput
+// x cache output to the paths that stopped at bounce b.
+__global__ void __launch_bounds__(kShadeThreads, kShadeMinBlocks)
+    wf_shade_nrc(const __grid_constant__ SingleWave w, WfState st, uint32_t b, const __grid_constant__ NrcWave nrc) {
+    shade_body<SingleWave, true>(w, st, b, &nrc);
+}
 __global__ void __launch_bounds__(128) wf_finish_nrc(const __grid_constant__ SingleWave w, WfState st,
                                                      const __grid_constant__ NrcWave nrc) {
     finish_body<SingleWave, true>(w, st, blockIdx.x * blockDim.x + threadIdx.x, &nrc);
@@ -91,7 +95,7 @@ cudaError_t grids(Grid& g) {
     int sms = 0, be = 0, bs = 0, bh = 0;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&be, wf_extend<kTraceWide>, 128, 0)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bs, shade_full_kernel(false), kShadeThreads, 0)) != cudaSuccess)
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bs, shade_full_kernel(), kShadeThreads, 0)) != cudaSuccess)
         return e;
     int bp = 0;
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bp, wf_shade_plain, kShadePlainThreads, 0)) != cudaSuccess)
@@ -207,7 +211,7 @@ cudaError_t launch_wavefront(const DevScene& s, const gbrt_ubo& ubo, const Rende
     J.path0 = 0;
     const int mode = trace_mode(s) | (s.all_opaque || ubo.fully_opaque ? kTraceOpaque : 0);
     // the shade form: the scene's material features and this frame's debug settings
-    const uint32_t feat = s.shade_feat | (ubo.mapping != 0u || ubo.debug == 1u ? kFeatDebug : 0u);
+    const uint32_t feat = job_features(s, ubo);
     // waves: k samples of a pixel range, k * npw <= cap
     for (uint32_t px0 = 0; px0 < npix;) {
         const uint32_t npw = npix - px0 < cap ? npix - px0 : cap;
@@ -236,7 +240,8 @@ cudaError_t launch_wavefront(const DevScene& s, const gbrt_ubo& ubo, const Rende
                 te();
                 if (side && b > 0 && (e = cudaStreamWaitEvent(stream, side->shadowed, 0)) != cudaSuccess) return e;
                 tb(1);
-                if (nrc || feat) launch_shade_full(w, st, b, nrc, bs, ts, stream);
+                if (nrc) wf_shade_nrc<<<bs, ts, 0, stream>>>(w, st, b, *nrc);
+                else if (feat) launch_shade_full(w, st, b, bs, ts, stream);
                 else wf_shade_plain<<<bp, tp, 0, stream>>>(w, st, b);
                 te();
                 if (nrc && !nrc->disabled && (nrc->mode == 1u ? b == 0 : b >= 1)) {  // queries of the paths that stopped here

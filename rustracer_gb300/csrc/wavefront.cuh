@@ -148,7 +148,14 @@ constexpr int kQueue = 0;     // [kQueue + b]: extension-queue length at bounce 
 constexpr int kShadow = 32;   // [kShadow + b]: shadow-queue length at bounce b
 constexpr int kWorkExt = 64;  // [kWorkExt + b]: fetch cursor of extend(b)
 constexpr int kWorkSh = 96;   // [kWorkSh + b]: fetch cursor of shadow(b)
+constexpr int kWorkShade = 128;  // [kWorkShade + b]: chunk cursor of shade(b) in batched waves
 constexpr int kMaxBounces = 31;
+
+// The material features a job's shading needs: its scene's, and debug shading
+// when its UBO asks for it.
+GB_HD uint32_t job_features(const DevScene& s, const gbrt_ubo& u) {
+    return s.shade_feat | (u.mapping != 0u || u.debug == 1u ? kFeatDebug : 0u);
+}
 constexpr uint32_t kPidMask = kMaxWavePaths - 1u;
 
 // Rows of a band of the pixel order.  Against row-major pixels with the
@@ -312,21 +319,21 @@ GB_D uint32_t nrc_train_hash(uint32_t pix, uint32_t sample) {
     return h & 0xFFFFu;
 }
 
+//
+// Shades the queue entries first, first + 1, ... below `last`, a block's width
+// of them at a time, `stride` apart.
 template <class Wv, bool kNrc = false, uint32_t kFeat = kFeatAll>
-GB_D void shade_body(const Wv& w, const WfState& st, uint32_t b, const NrcWave* nrc = nullptr) {
-    const uint32_t jb = w.block_job(1);
+GB_D void shade_range(const Wv& w, const WfState& st, uint32_t b, uint32_t jb, uint32_t first, uint32_t n,
+                      uint32_t stride, PathStats& ps, const NrcWave* nrc = nullptr) {
     const WaveJob& J = w.job(jb);
     const DevScene& s = J.s;
     const gbrt_ubo& ubo = J.ubo;
     uint32_t* cnt = st.counts + jb * kWfCounters;
-    const uint32_t n = cnt[kQueue + b], R = J.path0;
+    const uint32_t R = J.path0;
     const float4* __restrict__ rd = st.ray_d[b & 1] + R;
     float4* no = st.ray_o[(b + 1) & 1] + R;
     float4* nd = st.ray_d[(b + 1) & 1] + R;
     const uint32_t nb = ubo.number_of_bounces;
-    PathStats ps{0, 0, 0, 0, 0};
-    const uint32_t blk0 = w.blk0(1, jb), nblk = w.nblk(1, jb);
-    const uint32_t stride = nblk * blockDim.x;
     const bool sort_rays = s.sort_rays != 0u;
     __shared__ uint32_t s_key[2][34];
     uint32_t parity = 0;
@@ -335,7 +342,7 @@ GB_D void shade_body(const Wv& w, const WfState& st, uint32_t b, const NrcWave* 
         __syncthreads();
     }
     // block-uniform trip count (block_append2_by_key synchronises the block)
-    for (uint32_t cbase = (blockIdx.x - blk0) * blockDim.x; cbase < n; cbase += stride) {
+    for (uint32_t cbase = first; cbase < n; cbase += stride) {
         const uint32_t q = cbase + threadIdx.x;
         const bool active = q < n;
         bool cont = false, shadow = false;
@@ -507,8 +514,21 @@ GB_D void shade_body(const Wv& w, const WfState& st, uint32_t b, const NrcWave* 
             }
         }
     }
+}
+
+GB_D void flush_shade_stats(const PathStats& ps, DeviceCounters* c) {
     const unsigned long long hs = warp_sum<unsigned long long>(ps.shaded);
-    if (lane_id() == 0 && hs) atomicAdd(&J.out.counters->shaded, hs);
+    if (lane_id() == 0 && hs) atomicAdd(&c->shaded, hs);
+}
+
+// The whole queue of bounce b, its chunks dealt out in turn to the job's blocks.
+template <class Wv, bool kNrc = false, uint32_t kFeat = kFeatAll>
+GB_D void shade_body(const Wv& w, const WfState& st, uint32_t b, const NrcWave* nrc = nullptr) {
+    const uint32_t jb = w.block_job(1);
+    PathStats ps{0, 0, 0, 0, 0};
+    shade_range<Wv, kNrc, kFeat>(w, st, b, jb, (blockIdx.x - w.blk0(1, jb)) * blockDim.x,
+                                 st.counts[jb * kWfCounters + kQueue + b], w.nblk(1, jb) * blockDim.x, ps, nrc);
+    flush_shade_stats(ps, w.job(jb).out.counters);
 }
 
 // Any-hit shadow rays of bounce b (castShadowRay, RayTracing.rchit:35-59),
