@@ -81,6 +81,29 @@ struct Scratch {
     uint32_t *p_cnt, *p_pre, *p_off, *p_loff, *p_tile, *p_state;
 };
 
+// Adds a centroid of every thread with ok to the bounds cb: over the warp, the
+// block, then six atomics a block (per warp they took most of tri_boxes_kernel:
+// 48.8 -> 21 us for 327,714 triangles).
+__device__ __forceinline__ void add_centroid(bool ok, float3 c, uint32_t* cb) {
+    __shared__ uint32_t s_cb[6];
+    if (threadIdx.x < 6) s_cb[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
+    __syncthreads();
+    const float v[3] = {c.x, c.y, c.z};
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const bool in = ok && v[a] == v[a];  // a NaN does not count
+        const uint32_t mn = __reduce_min_sync(0xFFFFFFFFu, f2o(in ? v[a] : FLT_MAX));
+        const uint32_t mx = __reduce_max_sync(0xFFFFFFFFu, f2o(in ? v[a] : -FLT_MAX));
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&s_cb[a], mn);
+            atomicMax(&s_cb[3 + a], mx);
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < 3) atomicMin(cb + threadIdx.x, s_cb[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(cb + threadIdx.x, s_cb[threadIdx.x]);
+}
+
 // Item i's triangle (world space when `inst` is given and the item's
 // instance is a flattened transformed one), its box and TriRec.
 __global__ void tri_boxes_kernel(const gbrt_vertex* V, const uint32_t* I, const gbrt_priminfo* P, const uint4* items,
@@ -113,49 +136,13 @@ __global__ void tri_boxes_kernel(const gbrt_vertex* V, const uint32_t* I, const 
         unsorted[i] = r;
         c = (l + h) * 0.5f;
     }
-    // centroid bounds: warp reduce then atomics
-    float mnx = ok ? c.x : FLT_MAX, mny = ok ? c.y : FLT_MAX, mnz = ok ? c.z : FLT_MAX;
-    float mxx = ok ? c.x : -FLT_MAX, mxy = ok ? c.y : -FLT_MAX, mxz = ok ? c.z : -FLT_MAX;
-    for (int o = 16; o > 0; o >>= 1) {
-        mnx = fminf(mnx, __shfl_down_sync(0xFFFFFFFFu, mnx, o));
-        mny = fminf(mny, __shfl_down_sync(0xFFFFFFFFu, mny, o));
-        mnz = fminf(mnz, __shfl_down_sync(0xFFFFFFFFu, mnz, o));
-        mxx = fmaxf(mxx, __shfl_down_sync(0xFFFFFFFFu, mxx, o));
-        mxy = fmaxf(mxy, __shfl_down_sync(0xFFFFFFFFu, mxy, o));
-        mxz = fmaxf(mxz, __shfl_down_sync(0xFFFFFFFFu, mxz, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(cb + 0, f2o(mnx));
-        atomicMin(cb + 1, f2o(mny));
-        atomicMin(cb + 2, f2o(mnz));
-        atomicMax(cb + 3, f2o(mxx));
-        atomicMax(cb + 4, f2o(mxy));
-        atomicMax(cb + 5, f2o(mxz));
-    }
+    add_centroid(ok, c, cb);
 }
 
 __global__ void box_centroid_bounds_kernel(const float4* lo, const float4* hi, uint32_t n, uint32_t* cb) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool ok = i < n;
-    float3 c = ok ? (f3(lo[i]) + f3(hi[i])) * 0.5f : f3(0.0f);
-    float mnx = ok ? c.x : FLT_MAX, mny = ok ? c.y : FLT_MAX, mnz = ok ? c.z : FLT_MAX;
-    float mxx = ok ? c.x : -FLT_MAX, mxy = ok ? c.y : -FLT_MAX, mxz = ok ? c.z : -FLT_MAX;
-    for (int o = 16; o > 0; o >>= 1) {
-        mnx = fminf(mnx, __shfl_down_sync(0xFFFFFFFFu, mnx, o));
-        mny = fminf(mny, __shfl_down_sync(0xFFFFFFFFu, mny, o));
-        mnz = fminf(mnz, __shfl_down_sync(0xFFFFFFFFu, mnz, o));
-        mxx = fmaxf(mxx, __shfl_down_sync(0xFFFFFFFFu, mxx, o));
-        mxy = fmaxf(mxy, __shfl_down_sync(0xFFFFFFFFu, mxy, o));
-        mxz = fmaxf(mxz, __shfl_down_sync(0xFFFFFFFFu, mxz, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMin(cb + 0, f2o(mnx));
-        atomicMin(cb + 1, f2o(mny));
-        atomicMin(cb + 2, f2o(mnz));
-        atomicMax(cb + 3, f2o(mxx));
-        atomicMax(cb + 4, f2o(mxy));
-        atomicMax(cb + 5, f2o(mxz));
-    }
+    add_centroid(ok, ok ? (f3(lo[i]) + f3(hi[i])) * 0.5f : f3(0.0f), cb);
 }
 
 __global__ void morton_kernel(const float4* lo, const float4* hi, uint32_t n, const uint32_t* cb, uint32_t* codes,
