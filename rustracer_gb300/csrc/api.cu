@@ -193,7 +193,8 @@ int build_all(gbrt_scene* s) {
     cudaStream_t st = c->stream;
     const size_t ninst = s->instances.size();
     std::vector<DevInstance> hinst(ninst);
-    std::vector<uint4> world_items;
+    std::vector<uint4> world_spans;  // the world BVH's triangles: first item, instance, geometry, opaque
+    size_t nw = 0;
     std::vector<uint32_t> tlas_ids;
     std::vector<uint8_t> blas_needed(s->ngeo, 0);
     bool all_opaque = true;
@@ -231,8 +232,8 @@ int build_all(gbrt_scene* s) {
         if ((d.mask & 0xFFu) == 0 || ntri == 0) continue;
         if (!r.opaque) all_opaque = false;
         if (d.identity || flatten) {
-            for (uint32_t p = 0; p < ntri; ++p)
-                world_items.push_back(make_uint4((uint32_t)i, d.blas_geo, p, r.opaque ? 1u : 0u));
+            world_spans.push_back(make_uint4((uint32_t)nw, (uint32_t)i, d.blas_geo, r.opaque ? 1u : 0u));
+            nw += ntri;
         } else {
             blas_needed[d.blas_geo] = 1;
             tlas_ids.push_back((uint32_t)i);
@@ -244,7 +245,7 @@ int build_all(gbrt_scene* s) {
         nnodes += n > 1 ? n - 1 : 0;
         ntris += n;
     };
-    add(world_items.size());
+    add(nw);
     std::vector<uint32_t> blas_node_base(s->ngeo, 0), blas_tri_base(s->ngeo, 0);
     for (uint32_t g = 0; g < s->ngeo; ++g) {
         if (!blas_needed[g]) continue;
@@ -266,10 +267,12 @@ int build_all(gbrt_scene* s) {
     CU(c, upload(s->inst, hinst.data(), hinst.size(), st), "upload(instances)");
     if (hinst.empty()) CU(c, s->inst.alloc(sizeof(DevInstance)), "cudaMalloc");
     // world BVH
-    if (!world_items.empty()) {
-        CU(c, upload(s->items, world_items.data(), world_items.size(), st), "upload(items)");
+    if (nw) {
+        CU(c, upload(s->spans, world_spans.data(), world_spans.size(), st), "upload(spans)");
+        CU(c, s->items.alloc(nw * sizeof(uint4)), "cudaMalloc(items)");
+        CU(c, expand_spans(s->spans.as<uint4>(), (uint32_t)world_spans.size(), (uint32_t)nw, s->items.as<uint4>(), st),
+           "triangle items");
         BvhResult r;
-        const size_t nw = world_items.size();
         CU(c, s->cw_nodes.alloc(nw * sizeof(CwNode)), "cudaMalloc(wide nodes)");
         CU(c, s->cw_tris.alloc(nw * sizeof(TriRec)), "cudaMalloc(wide triangles)");
         const WideBuild wide{s->cw_nodes.as<CwNode>(), s->cw_tris.as<TriRec>(), &s->cw_count, &s->cw_levels, cw_width(s),
@@ -313,9 +316,10 @@ int build_all(gbrt_scene* s) {
         for (uint32_t g = 0; g < s->ngeo; ++g) {
             if (!blas_needed[g]) continue;
             const uint32_t ntri = s->ranges[g].i_len / 3;
-            std::vector<uint4> items(ntri);
-            for (uint32_t p = 0; p < ntri; ++p) items[p] = make_uint4(0u, g, p, s->ranges[g].opaque ? 1u : 0u);
-            CU(c, upload(bitems, items.data(), items.size(), st), "upload(blas items)");
+            const uint4 span = make_uint4(0u, 0u, g, s->ranges[g].opaque ? 1u : 0u);
+            CU(c, upload(s->spans, &span, 1, st), "upload(blas span)");
+            CU(c, bitems.reserve(ntri * sizeof(uint4)), "cudaMalloc(blas items)");
+            CU(c, expand_spans(s->spans.as<uint4>(), 1u, ntri, bitems.as<uint4>(), st), "triangle items");
             BvhResult r;
             uint32_t used = 0;
             const WideBuild wide{s->blas_cw_nodes.as<CwNode>() + cw_node0[g], s->blas_cw_tris.as<TriRec>() + cw_tri0[g],

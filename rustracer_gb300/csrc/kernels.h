@@ -235,6 +235,10 @@ struct WideBuild {
     double* sah;
 };
 
+// Items of whole geometries: span k (first item, instance id, geometry id,
+// opaque flag; first items ascending from 0) gives items first_k .. first_k+1.
+cudaError_t expand_spans(const uint4* spans, uint32_t nspans, uint32_t n, uint4* items, cudaStream_t st);
+
 // Item descriptors for triangle BVHs: x = instance id (world BVH) or 0,
 // y = BLAS geometry id, z = primitive id, w = opaque flag.
 // inst (may be null): items whose instance is not an identity one are

@@ -31,3 +31,26 @@ def test_build_order_of_sizes(gpu_ctx):
         sc = gbrt.Scene(gpu_ctx, sd)
         sc.create_top_as()
         assert_hits_equal(sc.trace(rays)[0], oracle_scene(sd).trace(rays)[0])
+
+
+@pytest.mark.parametrize("flags", [0, 1], ids=["flattened", "tlas"])
+def test_build_many_geometries(gpu_ctx, flags):
+    """Triangles of many geometries of one to forty triangles, in instances out of
+    order, repeated and masked out: each hit names its instance, geometry and primitive."""
+    import pyoracle as O
+    from rustracer_gb300 import gbrt
+    rng = np.random.default_rng(11)
+    b = scenes.GeoBuilder()
+    mat = b.add_material(scenes.random_pbr_material(rng))
+    for n in [1, 40, 2, 1, 31, 32, 33, 7]:
+        p = (rng.uniform(-1, 1, (n, 1, 3)) + rng.normal(0, 0.15, (n, 3, 3))).reshape(-1, 3).astype(np.float32)
+        b.add_mesh(p, np.arange(3 * n), mat, normal=np.tile(np.float32([0, 0, 1]), (3 * n, 1)))
+    order = [7, 0, 3, 5, 1, 5, 2, 6, 4, 0]
+    shift = [np.float32([1, 0, 0, x, 0, 1, 0, 0, 0, 0, 1, 0]) for x in (0, 0, .5, 0, 0, -.3, .2, 0, 0, .7)]
+    sd = b.finish(instances=scenes.identity_instances(order, shift),
+                  camera=dict(eye=(0, 0, 3.0), direction=(0, 0, -1), fov_deg=60.0))
+    sd.instances[3]["custom_index_and_mask"] &= 0xFFFFFF
+    rays = scenes.random_rays(20_000, seed=12)
+    ref = O.OracleScene(sd, build_flags=flags).trace(rays)[0]
+    assert len(np.unique(ref["instance_id"])) >= 8
+    assert_hits_equal(gbrt.Scene(gpu_ctx, sd, build_flags=flags).trace(rays)[0], ref)
