@@ -474,19 +474,27 @@ int refit_world(gbrt_scene* s) {
     // transformed instances (BLAS boxes feed the TLAS) or no 8-wide copy: full rebuild
     if (v.has_tlas || !v.has_world || !s->cw_count || s->cw_levels.size() < 2) return build_all(s);
     cudaStream_t st = c->stream;
-    // binary world BVH: rebuilt (an LBVH over the same items, one launch chain);
-    // 8-wide world BVH: refit in place, keeping its topology and slots
-    BvhResult r;
-    CU(c, build_triangle_bvh(c->build, s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
-                             s->prims.as<gbrt_priminfo>(), s->items.as<uint4>(), s->nworld, s->nodes.as<BNode2>(), 0, s->tris.as<TriRec>(), 0, &r,
-                             st, s->inst.as<DevInstance>(), kBvhFast),
-       "rebuild world BVH");
+    // binary and 8-wide world BVH: refit in place, keeping topology and slots (a
+    // binary one of a single leaf has no boxes: built again)
+    BvhResult r{};
+    const bool leaf = v.world_root < 0;
+    if (leaf)
+        CU(c, build_triangle_bvh(c->build, s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
+                                 s->prims.as<gbrt_priminfo>(), s->items.as<uint4>(), s->nworld, s->nodes.as<BNode2>(),
+                                 0, s->tris.as<TriRec>(), 0, &r, st, s->inst.as<DevInstance>(), kBvhFast),
+           "rebuild world BVH");
+    else
+        CU(c, refit_triangle_bvh(s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(),
+                                 s->prims.as<gbrt_priminfo>(), s->nodes.as<BNode2>(), s->tris.as<TriRec>(), s->nworld,
+                                 st, s->inst.as<DevInstance>()),
+           "refit world BVH");
     CU(c, s->cw_boxes.reserve((size_t)s->cw_count * 2 * sizeof(float4) + 16), "cudaMalloc(refit boxes)");
     double sah = 0.0;
     CU(c, refit_triangle_cwbvh(s->vertices.as<gbrt_vertex>(), s->indices.as<uint32_t>(), s->prims.as<gbrt_priminfo>(),
                                s->cw_nodes.as<CwNode>(), s->cw_tris.as<TriRec>(), s->nworld, s->cw_levels,
                                s->cw_boxes.as<float4>(), st, s->inst.as<DevInstance>(), &sah),
        "refit wide world BVH");
+    if (!leaf) CU(c, read_root(s->nodes.as<BNode2>(), &r, st), "read the root box");
     ++s->refits;
     s->cw_sah = sah;
     // topology kept through large deformations loses quality: rebuild once the tree's SAH cost proxy has

@@ -277,6 +277,14 @@ cudaError_t build_triangle_bvh_scratch(const BuildScratch& scratch, const gbrt_v
                                        uint32_t n, BNode2* nodes, uint32_t node_base, TriRec* tris,
                                        uint32_t tri_base, BvhResult* result_host, cudaStream_t st);
 
+// Refit of a binary BVH built by build_triangle_bvh over the same triangles at
+// node and triangle base 0, its root an inner node: records re-read from the
+// vertices, every node's boxes made again.  read_root waits for it and gives
+// the root (node 0) and its box.
+cudaError_t refit_triangle_bvh(const gbrt_vertex* vertices, const uint32_t* indices, const gbrt_priminfo* prims,
+                               BNode2* nodes, TriRec* tris, uint32_t n, cudaStream_t st, const DevInstance* inst);
+cudaError_t read_root(const BNode2* nodes, BvhResult* result_host, cudaStream_t st);
+
 // Refit of an 8-wide BVH built by build_triangle_bvh over the same
 // triangles: triangle records re-read from the vertices, then every node's
 // grid and child boxes recomputed level by level (level_starts: first node

@@ -23,7 +23,8 @@ struct alignas(16) BNode2 {
     float4 lxy;   // child 0: lo.x hi.x lo.y hi.y
     float4 rxy;   // child 1: lo.x hi.x lo.y hi.y
     float4 lrz;   // child 0: lo.z hi.z, child 1: lo.z hi.z
-    int4 c;       // c.x child 0, c.y child 1, c.z/c.w unused
+    int4 c;       // c.x child 0, c.y child 1; for refits: c.z parent * 2 + side
+                  // (-1 the root, -2 inside a leaf's range), c.w boxes arrived
 };
 static_assert(sizeof(BNode2) == 64, "BNode2 is 64 B");
 

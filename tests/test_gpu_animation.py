@@ -147,3 +147,30 @@ def test_gltf_keyframe_animation(gpu_ctx, tmp_path):
         assert_hits_equal(hits, ref)
     assert not np.array_equal(moved[0], moved[1])  # the animation moved something
     assert sc.info()["instance_updates"] >= 1
+
+
+@pytest.mark.parametrize("ntri", [1, 3, 5, 150, 3000])
+def test_refit_of_every_layout(gpu_ctx, ntri):
+    """Two instances that move twice: from worlds of one leaf to many tiles, the
+    8-wide and the binary tree give the oracle's hits."""
+    import pyoracle as O
+    from rustracer_gb300 import gbrt
+    sd = scenes.random_soup(ntri, seed=ntri, extent=0.4, size=0.15, nmat=1)
+
+    def instances(t):
+        c, s = np.cos(t), np.sin(t)
+        return scenes.identity_instances([0, 0], [np.float32([c, -s, 0, t, s, c, 0, 0, 0, 0, 1, 0]),
+                                                  np.float32([1, 0, 0, -t, 0, 1, 0, 0, 0, 0, 1, t])])
+
+    sd.instances = instances(0.2)
+    sc = gbrt.Scene(gpu_ctx, sd)
+    orc = O.OracleScene(sd)
+    rays = scenes.random_rays(5000, seed=5)
+    for t in (0.25, 0.4):
+        sc.update_tlas(instances(t))
+        orc.tlas(instances(t))
+        ref = orc.trace(rays)[0]
+        for width in (8, 2):  # neither builds anything again
+            sc.set_tuning(width)
+            assert_hits_equal(sc.trace(rays)[0], ref)
+    assert sc.info()["instance_updates"] == 2
