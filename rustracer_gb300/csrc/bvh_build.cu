@@ -17,6 +17,7 @@
 #include <utility>
 #include <float.h>
 #include "kernels.h"
+#include "launch.cuh"
 
 namespace gbrt {
 

@@ -9,12 +9,13 @@ namespace gbrt {
 
 __global__ void __launch_bounds__(kShadeThreads, kShadeMinBlocks)
     wf_shade(const __grid_constant__ SingleWave w, WfState st, uint32_t b) {
+    after_previous();
     shade_body<SingleWave, false, kFeatAll>(w, st, b);
 }
 
 void launch_shade_full(const SingleWave& w, const WfState& st, uint32_t b, uint32_t blocks, uint32_t threads,
                        cudaStream_t stream) {
-    wf_shade<<<blocks, threads, 0, stream>>>(w, st, b);
+    launch_after(wf_shade, blocks, threads, stream, w, st, b);
 }
 
 const void* shade_full_kernel() { return reinterpret_cast<const void*>(wf_shade); }

@@ -1,6 +1,7 @@
 // single_wave.cuh — the wave of a single frame: one job, one segment, passed to
 // the kernels as a __grid_constant__ parameter (wavefront.cu, shade_full.cu).
 #pragma once
+#include "launch.cuh"
 #include "wavefront.cuh"
 
 namespace gbrt {

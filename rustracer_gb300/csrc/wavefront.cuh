@@ -35,19 +35,28 @@ constexpr int trace_minb(int) { return GBRT_TRACE_MINB; }
 
 // Launches traversal kernel K in the form `mode` (trace_mode, with
 // kTraceOpaque when nothing in the launch can need the alpha test).
-#define GBRT_TRACE_LAUNCH(K, grid, threads, strm, ...)                                              \
-    switch (mode) {                                                                                 \
-        case kTraceWide: K<kTraceWide><<<grid, threads, 0, strm>>>(__VA_ARGS__); break;             \
-        case kTraceWideTlas: K<kTraceWideTlas><<<grid, threads, 0, strm>>>(__VA_ARGS__); break;     \
-        case kTraceBinary: K<kTraceBinary><<<grid, threads, 0, strm>>>(__VA_ARGS__); break;         \
-        case kTraceWide | kTraceOpaque:                                                             \
-            K<kTraceWide | kTraceOpaque><<<grid, threads, 0, strm>>>(__VA_ARGS__);                  \
-            break;                                                                                  \
-        case kTraceWideTlas | kTraceOpaque:                                                         \
-            K<kTraceWideTlas | kTraceOpaque><<<grid, threads, 0, strm>>>(__VA_ARGS__);              \
-            break;                                                                                  \
-        default: K<kTraceBinary | kTraceOpaque><<<grid, threads, 0, strm>>>(__VA_ARGS__); break;    \
+#define GBRT_TRACE_LAUNCH(K, grid, threads, strm, ...)                                          \
+    switch (mode) {                                                                             \
+        case kTraceWide: K<kTraceWide><<<grid, threads, 0, strm>>>(__VA_ARGS__); break;         \
+        case kTraceWideTlas: K<kTraceWideTlas><<<grid, threads, 0, strm>>>(__VA_ARGS__); break; \
+        case kTraceBinary: K<kTraceBinary><<<grid, threads, 0, strm>>>(__VA_ARGS__); break;     \
+        case kTraceWide | kTraceOpaque:                                                         \
+            K<kTraceWide | kTraceOpaque><<<grid, threads, 0, strm>>>(__VA_ARGS__);              \
+            break;                                                                              \
+        case kTraceWideTlas | kTraceOpaque:                                                     \
+            K<kTraceWideTlas | kTraceOpaque><<<grid, threads, 0, strm>>>(__VA_ARGS__);          \
+            break;                                                                              \
+        default: K<kTraceBinary | kTraceOpaque><<<grid, threads, 0, strm>>>(__VA_ARGS__); break; \
     }
+
+// The kernel of form `mode` for launch_after.
+#define GBRT_TRACE_KERNEL(K)                                                       \
+    (mode == kTraceWide                         ? K<kTraceWide>                    \
+     : mode == kTraceWideTlas                   ? K<kTraceWideTlas>                \
+     : mode == kTraceBinary                     ? K<kTraceBinary>                  \
+     : mode == (kTraceWide | kTraceOpaque)      ? K<kTraceWide | kTraceOpaque>     \
+     : mode == (kTraceWideTlas | kTraceOpaque)  ? K<kTraceWideTlas | kTraceOpaque> \
+                                                : K<kTraceBinary | kTraceOpaque>)
 
 // With the ray-sort key, shadow rays are grouped by octant too; shade blocks
 // of 256 threads make the groups twice as long (icosphere frame: 3719 Mrays/s
