@@ -166,8 +166,8 @@ const gbrt::NrcView& nrc_view(const gbrt_nrc* r);
 // One frame rendered with the cache into out, then its training steps
 // (gbrt_render_nrc without the host copies); *what names a failed step.
 cudaError_t nrc_frame(gbrt_nrc* r, const DevScene& view, const gbrt_ubo& ubo, const gbrt::RenderOut& out,
-                      const WfState& wf, const gbrt_nrc_render_opts& opts, cudaStream_t st, float* loss,
-                      const char** what);
+                      const WfState& wf, const gbrt_nrc_render_opts& opts, const gbrt::WfSide& side,
+                      cudaStream_t st, float* loss, const char** what);
 // The cache's query status word (0: no tensor-core wait has timed out); waits for st.
 uint32_t nrc_status(gbrt_nrc* r, cudaStream_t st);
 gbrt_ctx* nrc_ctx(const gbrt_nrc* r);

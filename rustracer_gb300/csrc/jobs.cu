@@ -340,7 +340,7 @@ int JobQueue::run_cache_job(Job* j, std::unique_lock<std::mutex>& lk) {
     wf.frame_sum = j->frame_sum.as<float4>();
     const char* what = "";
     lk.unlock();
-    cudaError_t e = nrc_frame(j->cache, j->scene->view, j->ubo, out, wf, j->copts, ctx->stream, nullptr, &what);
+    cudaError_t e = nrc_frame(j->cache, j->scene->view, j->ubo, out, wf, j->copts, ctx->side, ctx->stream, nullptr, &what);
     const uint32_t qstatus = e == cudaSuccess ? nrc_status(j->cache, ctx->stream) : 0u;
     lk.lock();
     if (e == cudaSuccess && qstatus) {

@@ -1327,7 +1327,8 @@ namespace gbrt_host {
 // frame's training samples.  Host-synchronises once, for the number of
 // training samples.  *what names the failed step.
 cudaError_t nrc_frame(gbrt_nrc* r, const DevScene& view, const gbrt_ubo& ubo, const RenderOut& out, const WfState& wf,
-                      const gbrt_nrc_render_opts& opts, cudaStream_t st, float* loss, const char** what) {
+                      const gbrt_nrc_render_opts& opts, const WfSide& side, cudaStream_t st, float* loss,
+                      const char** what) {
     const uint64_t paths = (uint64_t)out.width * out.height * ubo.number_of_samples;
     const uint32_t cap = (uint32_t)std::min<uint64_t>(std::min<uint64_t>(paths, wf.cap), kMaxWavePaths);
     const uint32_t tmax = std::max<uint32_t>(opts.train_samples, 1u) * 2u;  // room for the hash's spread
@@ -1363,7 +1364,7 @@ cudaError_t nrc_frame(gbrt_nrc* r, const DevScene& view, const gbrt_ubo& ubo, co
     w.cap = cap;
     *what = "wavefront launch";
     if ((e = cudaMemsetAsync(nw.counts + 32, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-    if ((e = launch_wavefront(view, ubo, out, w, st, nullptr, &nw, r)) != cudaSuccess) return e;
+    if ((e = launch_wavefront(view, ubo, out, w, st, nullptr, &nw, r, &side)) != cudaSuccess) return e;
     uint32_t ntrain = 0;
     *what = "training sample count";
     if ((e = cudaMemcpyAsync(&ntrain, nw.counts + 32, 4, cudaMemcpyDeviceToHost, st)) != cudaSuccess) return e;
@@ -1426,7 +1427,7 @@ extern "C" int gbrt_render_nrc(gbrt_scene* s, gbrt_nrc* r, const gbrt_ubo* ubo, 
     CU(c, cudaEventRecord(c->ev0, st), "event");
     float lsum = 0.0f;
     const char* what = "";
-    CU(c, nrc_frame(r, s->view, *ubo, out, c->wf, *opts, st, &lsum, &what), what);
+    CU(c, nrc_frame(r, s->view, *ubo, out, c->wf, *opts, c->side, st, &lsum, &what), what);
     CU(c, cudaEventRecord(c->ev1, st), "event");
     if (out_rgba8) CU(c, cudaMemcpyAsync(out_rgba8, out.rgba8, npix * 4, cudaMemcpyDeviceToHost, st), "download image");
     DeviceCounters dc;

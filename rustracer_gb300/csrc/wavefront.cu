@@ -186,19 +186,20 @@ cudaError_t launch_resolve(const gbrt_ubo& ubo, const RenderOut& out, const floa
 cudaError_t launch_wavefront(const DevScene& s, const gbrt_ubo& ubo, const RenderOut& out, const WfState& st,
                              cudaStream_t stream, StageTimer* timer, const NrcWave* nrc, gbrt_nrc* cache,
                              const WfSide* side) {
-    // the overlap needs the stages' own events off and leaves the cache form serial
-    // (its apply step updates the radiance the shadow stage also updates)
-    // and without point lights no shadow ray is made, so there is nothing to overlap
-    // (Cornell box of 64 x 64 paths 164 us with the events, 154 without; with point
-    // lights 415 and 530 in the material zoo)
-    if (timer || nrc || s.np == 0) side = nullptr;
+    // The overlap needs the stages' own events off.  Without point lights no
+    // shadow ray is made and there is nothing to overlap (Cornell box of 64 x 64
+    // paths 164 us with the events, 154 without; with point lights 415 and 530 in
+    // the material zoo).  In the cache form the shadow stage starts after the
+    // apply step, which updates the same radiance.
+    if (timer || s.np == 0) side = nullptr;
     if (ubo.number_of_bounces > kMaxBounces) return cudaErrorInvalidValue;
     cudaError_t e = grids(g_grid);
     if (e != cudaSuccess) return e;
     const uint32_t W = out.width, H = out.height, npix = W * H, ns = ubo.number_of_samples;
     const uint32_t sbase = ubo.total_number_of_samples - ns, nb = ubo.number_of_bounces;
     const uint32_t cap = st.cap < kMaxWavePaths ? st.cap : kMaxWavePaths;
-    if ((e = cudaMemsetAsync(st.frame_sum, 0, (size_t)npix * sizeof(float4), stream)) != cudaSuccess) return e;
+    if (ns == 0 && (e = cudaMemsetAsync(st.frame_sum, 0, (size_t)npix * sizeof(float4), stream)) != cudaSuccess)
+        return e;  // otherwise the finish of the first samples writes it
     if (timer) timer->used = 0;
     auto tb = [&](int stage) {
         if (timer) {

@@ -598,7 +598,8 @@ GB_D void finish_body(const Wv& w, const WfState& st, uint32_t i, const NrcWave*
     const uint32_t li = i - sg.fin0;
     const uint2 xy = pixel_at(sg.px0 + li, J.out.width, J.out.height);
     const uint32_t pix = xy.y * J.out.width + xy.x;
-    float4 acc = J.frame_sum[pix];
+    // a frame's first samples begin the sum; later waves of it add to it
+    const float4 acc = sg.si0 ? J.frame_sum[pix] : f4(0.0f, 0.0f, 0.0f, 0.0f);
     float3 sum = f3(acc);
     float last_t = acc.w;
     for (uint32_t j = 0; j < sg.k; ++j) {
