@@ -4,12 +4,17 @@
 
 namespace gbrt {
 
+#ifndef GBRT_RAYS_MINB
+#define GBRT_RAYS_MINB 8
+#endif
 // traceRayEXT queries (gbrt_trace_rays) through the persistent traversal of
-// the world BVH in the layout the scene carries.
+// the world BVH in the layout the scene carries.  Bound by instruction issue at
+// a third of the lanes, as the frame's traversal, and compiled in its forms and
+// at its occupancy.
 template <bool kAny, int kMode>
-__global__ void __launch_bounds__(128) trace_rays_persistent(DevScene s, const gbrt_ray* rays, uint32_t n,
-                                                             uint32_t flags, gbrt_hit* hits, uint32_t* work,
-                                                             DeviceCounters* cnt) {
+__global__ void __launch_bounds__(128, GBRT_RAYS_MINB)
+    trace_rays_persistent(DevScene s, const gbrt_ray* rays, uint32_t n, uint32_t flags, gbrt_hit* hits, uint32_t* work,
+                          DeviceCounters* cnt) {
     TraceStats ts{0, 0, 0};
     world_trace<kAny, kMode, true>(
         s, n, work, flags, ts, gridDim.x * (blockDim.x >> 5),
@@ -41,31 +46,27 @@ cudaError_t init_rays_constants(const float* texel_lut) {
 cudaError_t launch_trace_rays_persistent(const DevScene& s, const gbrt_ray* rays, uint32_t n, uint32_t flags,
                                          gbrt_hit* hits, uint32_t* work, DeviceCounters* cnt, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    static int dev_cached = -1, resident = 0;  // blocks of the persistent kernel that fit the GPU
-    int dev = 0;
+    // The form: as the frame's (launch constants of persistent.cuh).  One form with
+    // the TLAS walk and the alpha test for every scene took 254 us for 1,500,001
+    // random closest hits on an opaque icosphere of 327,680 triangles, its own
+    // 176 (any hits 255 and 197; with alpha tests, material zoo, 367 and 266).  With
+    // 8, 7, 6 and 5 blocks per SM: 176, 183, 190 and 213.
+    using Kernel = void (*)(DevScene, const gbrt_ray*, uint32_t, uint32_t, gbrt_hit*, uint32_t*, DeviceCounters*);
+    static constexpr Kernel kernels[2][6] = {
+        {trace_rays_persistent<false, 0>, trace_rays_persistent<false, 1>, trace_rays_persistent<false, 2>,
+         trace_rays_persistent<false, 4>, trace_rays_persistent<false, 5>, trace_rays_persistent<false, 6>},
+        {trace_rays_persistent<true, 0>, trace_rays_persistent<true, 1>, trace_rays_persistent<true, 2>,
+         trace_rays_persistent<true, 4>, trace_rays_persistent<true, 5>, trace_rays_persistent<true, 6>}};
+    const int form = trace_mode(s) + (s.all_opaque || (flags & GBRT_RAY_OPAQUE) ? 3 : 0);
+    const Kernel kernel = kernels[flags & GBRT_RAY_TERMINATE_ON_FIRST ? 1 : 0][form];
+    int dev = 0, sms = 0, per = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    if (dev != dev_cached) {
-        int sms = 0, per = 0;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, trace_rays_persistent<false, kTraceWideTlas>, 128, 0)) !=
-            cudaSuccess)
-            return e;
-        resident = sms * (per > 0 ? per : 1);
-        dev_cached = dev;
-    }
+    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 128, 0)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(work, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
-    const TraceGrid g = trace_grid(resident, n);
-    const bool any = flags & GBRT_RAY_TERMINATE_ON_FIRST;
-    // ray queries use the 8-wide form with the TLAS (it skips the TLAS of
-    // scenes without one), or the binary form where the scene needs it
-    if (trace_mode(s) != kTraceBinary) {
-        if (any) trace_rays_persistent<true, kTraceWideTlas><<<g.blocks, g.threads, 0, st>>>(s, rays, n, flags, hits, work, cnt);
-        else trace_rays_persistent<false, kTraceWideTlas><<<g.blocks, g.threads, 0, st>>>(s, rays, n, flags, hits, work, cnt);
-    } else {
-        if (any) trace_rays_persistent<true, kTraceBinary><<<g.blocks, g.threads, 0, st>>>(s, rays, n, flags, hits, work, cnt);
-        else trace_rays_persistent<false, kTraceBinary><<<g.blocks, g.threads, 0, st>>>(s, rays, n, flags, hits, work, cnt);
-    }
+    const TraceGrid g = trace_grid(sms * (per > 0 ? per : 1), n);
+    kernel<<<g.blocks, g.threads, 0, st>>>(s, rays, n, flags, hits, work, cnt);
     return cudaGetLastError();
 }
 

@@ -57,3 +57,23 @@ def test_crowded_leaves(gpu_ctx, ntri, size, masked):
     assert_hits_equal(sc.trace(rays)[0], ref)
     any_hits = sc.trace(rays, 0x4)[0]
     assert np.array_equal(any_hits["instance_id"] == 0xFFFFFFFF, ref["instance_id"] == 0xFFFFFFFF)
+
+
+@pytest.mark.parametrize("form", ["flattened", "tlas", "binary"])
+@pytest.mark.parametrize("masked", [0.0, 0.5], ids=["opaque", "masked"])
+def test_ray_query_forms(gpu_ctx, form, masked):
+    """Closest and any hits, with and without the alpha test, through each form of the query kernel."""
+    import pyoracle as O
+    from rustracer_gb300 import gbrt
+    sd = scenes.random_soup(900, seed=17, extent=0.6, size=0.15, alpha_mask_fraction=masked)
+    sd.instances["transform"][1] = np.float32([0.8, 0, 0, 0.3, 0, 0.8, 0, 0, 0, 0, 0.8, -0.2])
+    build = gbrt.BUILD_NO_FLATTEN if form == "tlas" else 0
+    sc, orc = gbrt.Scene(gpu_ctx, sd, build_flags=build), O.OracleScene(sd, build_flags=build)
+    if form == "binary":
+        sc.set_tuning(2)
+    rays = scenes.random_rays(4097, seed=18)
+    for flags in (0, 1):  # GBRT_RAY_OPAQUE
+        ref = orc.trace(rays, flags)[0]
+        assert_hits_equal(sc.trace(rays, flags)[0], ref)
+        any_hit = sc.trace(rays, flags | 4)[0]  # GBRT_RAY_TERMINATE_ON_FIRST: some hit of the ray
+        assert np.array_equal(any_hit["t"] >= 0, ref["t"] >= 0)
