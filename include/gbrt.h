@@ -356,9 +356,8 @@ int gbrt_tlas_build(gbrt_scene* scene, const gbrt_instance* instances, uint32_t 
  * geometries, masks, custom indices and flags, and, for instances kept under
  * the TLAS, the same identity / non-identity class), the update is
  * incremental: transformed instances merged into the world BVH re-transform
- * their triangles, the binary world BVH is rebuilt with the fast Morton tree
- * and the wide one refit in place (a full build once the refit's SAH cost
- * proxy has drifted 1.3x); a TLAS is rebuilt over the instances' new world
+ * their triangles and both layouts of the world BVH are refit in place (a
+ * full build once the wide one's SAH cost proxy has drifted 1.3x); a TLAS is rebuilt over the instances' new world
  * boxes with the BLASes untouched.  Any other change takes a full build, as
  * gbrt_tlas_build.  Hits are the same as after gbrt_tlas_build with these
  * instances.  GBRT_E_BUSY while the context has unfinished jobs.

@@ -384,9 +384,8 @@ int build_all(gbrt_scene* s) {
 // gbrt_tlas_update: the instances keep their geometries, masks and custom
 // indices and only their transforms move (the reference's animated frames,
 // gltf_viewer main.rs:395-402 -> create_top_as).  Transformed instances merged
-// into the world BVH re-transform their triangles: the binary world BVH is
-// rebuilt (Morton radix tree, one launch chain) and the wide one refit in
-// place, with the refit's drift check; a TLAS is rebuilt over the instances'
+// into the world BVH re-transform their triangles: both layouts of it are
+// refit in place, with the refit's drift check; a TLAS is rebuilt over the instances'
 // new world boxes, the BLASes untouched.  Anything else changing (a geometry,
 // a mask, an instance entering or leaving the world BVH) takes a full build.
 int update_instances(gbrt_scene* s, const gbrt_instance* in, uint32_t n) {

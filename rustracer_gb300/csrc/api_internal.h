@@ -151,8 +151,8 @@ int build_all(gbrt_scene* s);
 // Linear-blend skinning of the scene's bind-pose vertices, then refit_world.
 int skin_scene(gbrt_scene* s, const gbrt_skin_raw* skins, uint32_t nskin);
 void fill_stats(gbrt_stats* st, const DeviceCounters& dc, double ms, uint32_t launches);
-// After the vertices moved: the binary world BVH rebuilt and the 8-wide one
-// refit in place (topology kept); scenes with transformed instances rebuild
+// After the vertices moved: the binary and the 8-wide world BVH refit in place
+// (topology kept); scenes with transformed instances rebuild
 // everything (build_all).
 int refit_world(gbrt_scene* s);
 

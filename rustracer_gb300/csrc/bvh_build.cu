@@ -2,7 +2,7 @@
 //
 // 30-bit Morton codes of the item centroids and a CUB radix sort, then a
 // binary tree: by default parallel locally-ordered clustering
-// (ploc_build.inc), or, for fast rebuilds, the linear BVH of Karras 2012
+// (ploc_build.inc), or, for allocation-free rebuilds, the linear BVH of Karras 2012
 // ("Maximizing Parallelism in the Construction of BVHs, Octrees, and k-d
 // Trees": one thread per inner node finds its key range and split); then one
 // bottom-up pass (atomic arrival counters) that computes the boxes

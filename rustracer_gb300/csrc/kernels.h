@@ -201,8 +201,7 @@ struct BvhResult {
 };
 
 // Binary-tree construction of the BVH builders: kBvhPloc clusters the items
-// (parallel locally-ordered clustering, better trees, a host wait per
-// round), kBvhFast splits the Morton order (Karras radix tree, one launch).
+// (parallel locally-ordered clustering, better trees, one host wait), kBvhFast splits the Morton order (Karras radix tree, one launch).
 constexpr int kBvhFast = 0, kBvhPloc = 1;
 
 // Device memory that the builds of a context carve their scratch from: grown
