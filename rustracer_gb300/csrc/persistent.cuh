@@ -116,7 +116,7 @@ GB_D void persistent_trace(const DevScene& s, uint32_t n, uint32_t* work, uint32
                 cur = kEmpty;
                 while (sp > 0) {
                     --sp;
-                    if (stack_t[sp] <= best.t) {
+                    if (stack_t[sp] <= best.t * kBoxSlack) {
                         cur = stack_node[sp];
                         break;
                     }
@@ -148,7 +148,7 @@ GB_D void persistent_trace(const DevScene& s, uint32_t n, uint32_t* work, uint32
                 cur = kEmpty;
                 while (sp > 0) {
                     --sp;
-                    if (stack_t[sp] <= best.t) {
+                    if (stack_t[sp] <= best.t * kBoxSlack) {
                         cur = stack_node[sp];
                         break;
                     }

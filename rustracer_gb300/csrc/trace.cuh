@@ -93,10 +93,16 @@ GB_D bool isect_tri(const TRay& r, float3 p0, float3 p1, float3 p2, float tmin, 
     return true;
 }
 
+// Rounding of slab distances: 1 + 2*gamma(3), gamma(n) = n*2^-24 / (1 - n*2^-24).
+// A box is out of a hit's reach when its entry distance is beyond t * kBoxSlack;
+// one put aside is held to the same limit again when its turn comes, so that a
+// tie in t (two triangles in one plane, each in a flat box) is found either way.
+constexpr float kBoxSlack = 1.0000003576278687f;
+
 // Robust slab test against [lo, hi]; returns the entry distance in tn.
 GB_D bool box_hit(const TRay& r, float lox, float hix, float loy, float hiy, float loz, float hiz, float tmin,
                   float tcur, float& tn) {
-    const float up = 1.0000003576278687f;  // 1 + 2*gamma(3), gamma(n) = n*2^-24 / (1 - n*2^-24)
+    const float up = kBoxSlack;
     float t0x = (lox - r.o.x) * r.inv.x, t1x = (hix - r.o.x) * r.inv.x;
     float t0y = (loy - r.o.y) * r.inv.y, t1y = (hiy - r.o.y) * r.inv.y;
     float t0z = (loz - r.o.z) * r.inv.z, t1z = (hiz - r.o.z) * r.inv.z;

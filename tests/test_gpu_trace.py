@@ -181,3 +181,16 @@ def test_degenerate_layouts_build_and_match(gpu_ctx, layout):
     assert_hits_equal(hits, ref)
     assert st["device_status"] == 0
     assert (hits["instance_id"] != 0xFFFFFFFF).sum() > 100
+
+
+def test_binary_layout_ties(gpu_ctx):
+    """Boxes that stand on a floor: where a ray meets both planes at the same t, the
+    smaller (instance, primitive) wins in the binary layout too."""
+    from rustracer_gb300 import gbrt
+    sd = scenes.icosphere_scene(subdiv=3)
+    sc = gbrt.Scene(gpu_ctx, sd)
+    sc.set_tuning(2)
+    p = sd.vertices["pos"][:, :3]
+    rays = scenes.random_rays(200_000, seed=50)
+    rays["org"] = np.random.default_rng(51).uniform(p.min(0), p.max(0), (len(rays), 3)) - 2.0 * rays["dir"]
+    assert_hits_equal(sc.trace(rays)[0], oracle_scene(sd).trace(rays)[0])
