@@ -248,16 +248,23 @@ GB_D float2 cw_planes(uint32_t n0, uint32_t n1, uint32_t f0, uint32_t f1, int k,
     return t;
 }
 
-// A ray for the 8-wide form: inverses at most 2^96, so that an axis it is
-// parallel to (or as good as parallel: 2^-96 of a unit per unit of t) needs no
-// case of its own.  Its slab distances are then +-(distance to the plane) *
-// 2^96, which lie outside any query's [tmin, tmax] on the proper sides, or
-// NaN, which min and max pass over.
-constexpr float kCwInvMax = 7.9228162514264338e28f;
+// A ray for the 8-wide form: an axis it is parallel to needs no case of its own.
+// Its inverse there is 2^96, so its slab distances are +-(distance to the plane)
+// * 2^96, on the proper sides of any distance the ray can reach in the scene, or
+// NaN, which min and max pass over.  A direction shorter than 1 makes the
+// distances along its other axes longer, so the inverse grows with that of the
+// largest component, by powers of two (a node's grid step times it then rounds
+// nowhere and overflows to infinity alone); for directions below 2^-32 it is
+// infinite and the axis does not cull.  Components other than 0 keep their
+// inverse: near and far plane stay in proportion to the other axes.
+constexpr float kCwInvParallel = 7.9228162514264338e28f;
 GB_D void cw_ray(TRay& r) {
-    r.inv.x = clampf(r.inv.x, -kCwInvMax, kCwInvMax);
-    r.inv.y = clampf(r.inv.y, -kCwInvMax, kCwInvMax);
-    r.inv.z = clampf(r.inv.z, -kCwInvMax, kCwInvMax);
+    // r.Sz: inverse of the largest component; its power of two
+    const float most = kCwInvParallel * fmaxf(1.0f, __uint_as_float(__float_as_uint(r.Sz) & 0x7F800000u));
+    auto axis = [&](float d, float inv) { return fabsf(d) > 0.0f ? inv : copysignf(most, inv); };
+    r.inv.x = axis(r.d.x, r.inv.x);
+    r.inv.y = axis(r.d.y, r.inv.y);
+    r.inv.z = axis(r.d.z, r.inv.z);
 }
 
 // Intersects the 8 children of wide node `node`: returns the hit mask (bits

@@ -194,3 +194,37 @@ def test_binary_layout_ties(gpu_ctx):
     rays = scenes.random_rays(200_000, seed=50)
     rays["org"] = np.random.default_rng(51).uniform(p.min(0), p.max(0), (len(rays), 3)) - 2.0 * rays["dir"]
     assert_hits_equal(sc.trace(rays)[0], oracle_scene(sd).trace(rays)[0])
+
+
+def _parallel_rays(sd, n, length, zeros, seed):
+    """Rays along an axis (two zero components) or in a plane of two (one), of directions `length` long, at the scene."""
+    rng = np.random.default_rng(seed)
+    p = sd.vertices["pos"][:, :3]
+    d = np.zeros((n, 3), np.float32)
+    axis = rng.integers(0, 3, n)
+    d[np.arange(n), axis] = rng.choice(np.float32([-1, 1]), n)
+    if zeros == 1:
+        d[np.arange(n), (axis + 1) % 3] = rng.uniform(-1, 1, n)
+    r = scenes.random_rays(n, seed=seed, tmax=3e38)
+    r["org"] = rng.uniform(p.min(0), p.max(0), (n, 3)) - 2.0 * d
+    r["dir"] = d * np.float32(length)
+    return r
+
+
+@pytest.mark.parametrize("length", [1.0, 1e-9, 1e-12, 1e-20, 1e-27, 1e-34])
+def test_parallel_rays_of_any_length(gpu_ctx, length):
+    """Rays parallel to an axis hit what the oracle says whatever the length of
+    their direction, in every layout, in BLASes under a TLAS too."""
+    import pyoracle as O
+    from rustracer_gb300 import gbrt
+    for sd, flags in ((scenes.icosphere_scene(subdiv=4), 0), (_instanced_scene(), 1)):
+        sc, orc = gbrt.Scene(gpu_ctx, sd, build_flags=flags), O.OracleScene(sd, build_flags=flags)
+        for zeros in (1, 2):
+            rays = _parallel_rays(sd, 4000, length, zeros, seed=40 + zeros)
+            ref = orc.trace(rays)[0]
+            hit = ref["instance_id"] != 0xFFFFFFFF
+            assert hit.mean() > (0.99 if flags == 0 else 0.1)
+            for width in (8, 4, 2):
+                sc.set_tuning(width)
+                assert_hits_equal(sc.trace(rays)[0], ref)
+                assert np.array_equal(sc.trace(rays, 0x4)[0]["instance_id"] != 0xFFFFFFFF, hit)
