@@ -479,7 +479,7 @@ __global__ void init_bounds_kernel(uint32_t* cb) {
 
 inline uint32_t blocks(uint32_t n, uint32_t b = 256) { return (n + b - 1) / b; }
 
-// Lays the scratch of one build over n items out in the context's arena.
+// Lays the scratch of one build over n items out in the context's arena, which the build holds.
 cudaError_t scratch_carve(Scratch& s, uint32_t n, BuildArena& arena, cudaStream_t st) {
     std::memset(&s, 0, sizeof(s));
     const size_t m = n > 1 ? n - 1 : 1;
@@ -543,20 +543,6 @@ cudaError_t scratch_carve(Scratch& s, uint32_t n, BuildArena& arena, cudaStream_
 }
 
 }  // namespace
-
-cudaError_t BuildArena::reserve(size_t n) {
-    if (n <= bytes) return cudaSuccess;
-    release();
-    const cudaError_t e = cudaMalloc(&p, n);
-    if (e == cudaSuccess) bytes = n;
-    else p = nullptr;
-    return e;
-}
-void BuildArena::release() {
-    if (p) cudaFree(p);
-    p = nullptr;
-    bytes = 0;
-}
 
 #include "ploc_build.inc"
 
@@ -656,6 +642,7 @@ cudaError_t build_triangle_bvh(BuildArena& arena, const gbrt_vertex* vertices, c
                                uint32_t node_base, TriRec* tris, uint32_t tri_base, BvhResult* res, cudaStream_t st,
                                const DevInstance* inst, int quality, const WideBuild* wide) {
     if (n == 0 || (wide && (wide->width < 2 || wide->width > 8))) return cudaErrorInvalidValue;
+    std::lock_guard<std::mutex> hold(arena.mu);
     Scratch s;
     CK(scratch_carve(s, n, arena, st));
     init_bounds_kernel<<<1, 32, 0, st>>>(s.cbounds);
@@ -691,6 +678,7 @@ cudaError_t build_instance_bvh(BuildArena& arena, const float4* lo, const float4
                                BNode2* nodes, uint32_t node_base, TriRec* tris, uint32_t tri_base, BvhResult* res,
                                cudaStream_t st, int quality) {
     if (n == 0) return cudaErrorInvalidValue;
+    std::lock_guard<std::mutex> hold(arena.mu);
     Scratch s;
     CK(scratch_carve(s, n, arena, st));
     CK(cudaMemcpyAsync(s.lo, lo, n * sizeof(float4), cudaMemcpyDeviceToDevice, st));

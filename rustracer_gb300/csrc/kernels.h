@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <vector>
+#include "build_arena.h"
 #include "scene.cuh"
 
 namespace gbrt {
@@ -203,21 +204,6 @@ struct BvhResult {
 // Binary-tree construction of the BVH builders: kBvhPloc clusters the items
 // (parallel locally-ordered clustering, better trees, one host wait), kBvhFast splits the Morton order (Karras radix tree, one launch).
 constexpr int kBvhFast = 0, kBvhPloc = 1;
-
-// Device memory that the builds of a context carve their scratch from: grown
-// to the largest build's need (about 270 B per triangle) and kept, so that a
-// rebuild of an animated scene does not allocate.  One build at a time uses
-// it, in the order of the context's stream.
-struct BuildArena {
-    void* p = nullptr;
-    size_t bytes = 0;
-    BuildArena() = default;
-    BuildArena(const BuildArena&) = delete;
-    BuildArena& operator=(const BuildArena&) = delete;
-    ~BuildArena() { release(); }
-    cudaError_t reserve(size_t n);
-    void release();
-};
 
 // The compressed 8-wide form of a triangle BVH, built from the same binary
 // tree: nodes (capacity n, root at 0) and their triangles (n slots, node-leaf

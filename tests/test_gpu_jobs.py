@@ -322,3 +322,55 @@ def test_serving_skinned_job_vs_oracle(gpu_ctx):
     ref = orc.render(ubo, W, H, want_samples=True, want_hits=True, want_margins=True)
     assert np.array_equal(solo["hits"]["primitive_id"], ref["hits"]["primitive_id"])
     parity.assert_samples(solo["samples"], ref, orc, ubo, W, H)
+
+
+def test_builds_beside_skinned_jobs():
+    """The job worker rebuilds a skinned scene (its tube under a TLAS) while another
+    thread rebuilds a second scene of the same context: each gets its own trees."""
+    import threading
+    import pyoracle as O
+    from rustracer_gb300 import gbrt
+    from test_gpu_trace import assert_hits_equal
+    ctx = gbrt.Context(0)
+    sd = zoo.skinned_tube()
+    sd.instances["transform"][-1] = np.float32([1, 0, 0, 0.2, 0, 1, 0, 0, 0, 0, 1, 0])  # the tube
+    sc = gbrt.Scene(ctx, sd, build_flags=gbrt.BUILD_NO_FLATTEN)
+    ubo = sd.ubo(48, 48, samples=1, bounces=4, exposure=1.0)
+    skins = [zoo.bone_matrices(sd.bones, t) for t in (0.3, 0.9, 1.7)]
+    ref = []
+    for s in skins:
+        sc.skin_and_refit(s)
+        ref.append(_solo(ctx, sc, ubo, 48, 48)[1])
+    assert not np.array_equal(ref[0], ref[1])
+    other = scenes.icosphere_scene(subdiv=5)
+    rays = scenes.random_rays(2000, seed=3)
+    hits = O.OracleScene(other).trace(rays)[0]
+    sc2 = gbrt.Scene(ctx, other)
+    accs = [gbrt.Accum(ctx, 48, 48) for _ in range(120)]
+    stop, built, failed = threading.Event(), [0], []
+
+    def rebuild():
+        while not stop.is_set():
+            try:
+                sc2.create_top_as()
+                built[0] += 1
+                assert_hits_equal(sc2.trace(rays)[0], hits)
+            except gbrt.GbrtError as e:  # jobs are running
+                if e.code != gbrt.E_BUSY:
+                    failed.append(e)
+            except AssertionError as e:
+                failed.append(e)
+
+    th = threading.Thread(target=rebuild)
+    th.start()
+    try:
+        for i, acc in enumerate(accs):  # this thread: the job API alone
+            assert ctx.submit(sc, ubo, acc, skins=skins[i % 3]).wait()["status"] == 0
+    finally:
+        stop.set()
+        th.join()
+    assert not failed and built[0] > 0, (failed[:3], built)
+    for i, acc in enumerate(accs):
+        assert np.array_equal(acc.download(), ref[i % 3]), i
+    del sc, sc2, acc, accs
+    ctx.close()
