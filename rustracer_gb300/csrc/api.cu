@@ -182,10 +182,6 @@ void refresh_view(gbrt_scene* s) {
     v.blas_cw_tris = s->blas_cw_nodes.p ? s->blas_cw_tris.as<TriRec>() : nullptr;
 }
 
-// Build scratch that a context keeps between builds: scenes of up to four
-// million triangles rebuild without allocating, larger ones give theirs back.
-constexpr size_t kArenaKeep = size_t(1) << 30;
-
 // Builds the merged world BVH, the BLASes of transformed instances and the
 // TLAS into fresh pools.
 int build_all(gbrt_scene* s) {
@@ -256,6 +252,7 @@ int build_all(gbrt_scene* s) {
     const uint32_t tlas_node_base = (uint32_t)nnodes, tlas_tri_base = (uint32_t)ntris;
     add(tlas_ids.size());
     if (ntris >= (1u << 28)) return fail(c, GBRT_E_INVALID, "scene exceeds 2^28 leaf slots");
+    BuildCall call(c->build);
     CU(c, s->nodes.alloc(std::max<size_t>(1, nnodes) * sizeof(BNode2)), "cudaMalloc(nodes)");
     CU(c, s->tris.alloc(std::max<size_t>(1, ntris) * sizeof(TriRec)), "cudaMalloc(tris)");
     DevScene& v = s->view;
@@ -371,13 +368,13 @@ int build_all(gbrt_scene* s) {
         s->blas_cw_tris.release();
         CU(c, cudaStreamSynchronize(st), "sync after build");
     }
-    if (c->build.bytes > kArenaKeep) c->build.release();  // the stream has been waited for
     s->h_inst = std::move(hinst);
     s->tlas_ids = std::move(tlas_ids);
     s->flattened = false;
     for (const DevInstance& d : s->h_inst) s->flattened = s->flattened || (flatten && !d.identity && (d.mask & 0xFFu));
     refresh_view(s);
     s->built = v.has_world || v.has_tlas;
+    call.done();
     return GBRT_OK;
 }
 
@@ -413,6 +410,7 @@ int update_instances(gbrt_scene* s, const gbrt_instance* in, uint32_t n) {
        "upload(instances)");
     DevScene& v = s->view;
     if (v.has_tlas) {
+        BuildCall call(c->build);
         const uint32_t nt = (uint32_t)s->tlas_ids.size();
         CU(c, instance_world_boxes(s->inst.as<DevInstance>(), s->tlas_ids_d.as<uint32_t>(), s->tlas_blo.as<float4>(),
                                    s->tlas_bhi.as<float4>(), nt, s->tlas_lo.as<float4>(), s->tlas_hi.as<float4>(), st),
@@ -425,6 +423,7 @@ int update_instances(gbrt_scene* s, const gbrt_instance* in, uint32_t n) {
         v.tlas_root = r.root;
         v.tlas_lo = r.lo;
         v.tlas_hi = r.hi;
+        call.done();
     }
     ++s->instance_updates;
     if (s->flattened) return refit_world(s);

@@ -8,13 +8,15 @@
 
 namespace gbrt {
 
-// Grown to the largest build's need (about 270 B per triangle) and kept, so
-// that a rebuild of an animated scene does not allocate.  A build holds `mu`
+// Grown to the largest build's need (about 270 B per triangle) and kept up to
+// kKeep, so that a rebuild of an animated scene does not allocate: scenes of up
+// to four million triangles rebuild in it, larger ones give theirs back.  A build holds `mu`
 // from its reserve to its last launch: a context's builds come from the
 // caller's thread and, for skinned jobs, from the job worker's, each of many
 // launches with host waits between them, and their order on the stream keeps
 // two of them apart only when one is queued whole before the other.
 struct BuildArena {
+    static constexpr size_t kKeep = size_t(1) << 30;
     void* p = nullptr;
     size_t bytes = 0;
     std::mutex mu;
@@ -36,6 +38,24 @@ struct BuildArena {
         p = nullptr;
         bytes = 0;
     }
+    // Gives memory back beyond `keep` bytes.
+    void trim(size_t keep) {
+        std::lock_guard<std::mutex> hold(mu);
+        if (bytes > keep) release();
+    }
+};
+
+// The life of one call's builds: when it ends the arena keeps at most kKeep,
+// and nothing unless the call says done(), since a call that fails is likely
+// short of memory.
+struct BuildCall {
+    BuildArena& arena;
+    size_t keep = 0;
+    explicit BuildCall(BuildArena& a) : arena(a) {}
+    BuildCall(const BuildCall&) = delete;
+    BuildCall& operator=(const BuildCall&) = delete;
+    ~BuildCall() { arena.trim(keep); }
+    void done() { keep = BuildArena::kKeep; }
 };
 
 }  // namespace gbrt
