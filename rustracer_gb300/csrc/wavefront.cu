@@ -93,6 +93,7 @@ namespace {
 struct Grid {
     int dev = -1;
     int sms = 0, extend = 0, shade = 0, shade_plain = 0, shadow = 0;
+    int extend_binary = 0, shadow_binary = 0;  // the opaque binary form
 };
 Grid g_grid;
 
@@ -112,6 +113,15 @@ cudaError_t grids(Grid& g) {
     g.shade_plain = sms * (bp > 0 ? bp : 1);
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bh, wf_shadow<kTraceWide>, 128, 0)) != cudaSuccess) return e;
     g.extend = sms * (be > 0 ? be : 1);
+    int b2 = 0, h2 = 0;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b2, wf_extend<kTraceBinary | kTraceOpaque>, 128, 0)) !=
+        cudaSuccess)
+        return e;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&h2, wf_shadow<kTraceBinary | kTraceOpaque>, 128, 0)) !=
+        cudaSuccess)
+        return e;
+    g.extend_binary = sms * (b2 > 0 ? b2 : 1);
+    g.shadow_binary = sms * (h2 > 0 ? h2 : 1);
     g.shade = sms * (bs > 0 ? bs : 1);
     g.shadow = sms * (bh > 0 ? bh : 1);
     g.sms = sms;
@@ -240,7 +250,9 @@ cudaError_t launch_wavefront(const DevScene& s, const gbrt_ubo& ubo, const Rende
                 if ((e = cudaMemsetAsync(nrc->snap_pos, 0, (size_t)J.npaths * sizeof(float4), stream)) != cudaSuccess)
                     return e;
             }
-            const TraceGrid ge = trace_grid(g_grid.extend, J.npaths), gh = trace_grid(g_grid.shadow, J.npaths);
+            const bool binary = mode == (kTraceBinary | kTraceOpaque);  // other launch bounds (trace_minb)
+            const TraceGrid ge = trace_grid(binary ? g_grid.extend_binary : g_grid.extend, J.npaths),
+                            gh = trace_grid(binary ? g_grid.shadow_binary : g_grid.shadow, J.npaths);
             const uint32_t ts = shade_threads(J.npaths, kShadeThreads), tp = shade_threads(J.npaths, kShadePlainThreads);
             const uint32_t bs = shade_blocks(J.npaths, ts, g_grid.shade),
                            bp = shade_blocks(J.npaths, tp, g_grid.shade_plain);

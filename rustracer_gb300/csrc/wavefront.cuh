@@ -23,15 +23,21 @@
 
 // Resident 128-thread blocks per SM the traversal kernels (extend, shadow)
 // are compiled for: 8 gives them 64 registers, which the 8-wide forms need (no
-// spills without alpha tests, 20 B with them), at 32 warps per SM to cover
-// dependent node and triangle loads.  6 / 7 / 8 / 9 / 10 blocks: icosphere
-// frame (1080p x 64) 89.9 / 80.3 / 77.3 / 78.8 / 79.7 ms (6 on an earlier form),
-// instanced tori - / 11.6 / 11.4 / 12.3 / 13.5 ms.
+// spills without alpha tests, 20 to 28 B with them, 184 to 304 B with the TLAS),
+// at 32 warps per SM to cover dependent node and triangle loads.  6 / 7 / 8 / 9 /
+// 10 blocks: icosphere frame (1080p x 64) 89.9 / 80.3 / 77.3 / 78.8 / 79.7 ms (6 on
+// an earlier form), instanced tori - / 11.6 / 11.4 / 12.3 / 13.5 ms.
 #ifndef GBRT_TRACE_MINB
 #define GBRT_TRACE_MINB 8
 #endif
-// Same bound for every traversal form.
-constexpr int trace_minb(int) { return GBRT_TRACE_MINB; }
+// The opaque binary form runs at 7, where it spills little (72 registers; 72 to
+// 88 B of stores at 64): icosphere frames of 640 x 360 x 4 with 327,680 triangles
+// 1.96 -> 1.90 ms, 20,480 1.33 -> 1.29, 24 frames of 256 x 256 x 2 6.76 -> 6.67.  With
+// the alpha test 8 are better there too: instanced tori of 1280 x 720 x 8 15.6 ms
+// at 7, 15.3 at 8.
+constexpr int trace_minb(int mode) {
+    return mode == (gbrt::kTraceBinary | gbrt::kTraceOpaque) ? 7 : GBRT_TRACE_MINB;
+}
 
 // Launches traversal kernel K in the form `mode` (trace_mode, with
 // kTraceOpaque when nothing in the launch can need the alpha test).
