@@ -309,7 +309,7 @@ __global__ void bottom_up_kernel(int n, const uint32_t* idx, const float4* lo, c
             }
             const float leaf_cost = count <= kCwMaxLeaf ? kCwCostTri * a * (float)count : FLT_MAX;
             const float node_cost = kCwCostNode * a + all;
-            const bool leaf = leaf_cost <= node_cost;
+            const bool leaf = count <= kCwMaxLeaf && leaf_cost <= node_cost;  // an area can be infinite
             float v = leaf ? leaf_cost : node_cost;
             out[0] = v;
             best[0] = kall;

@@ -54,3 +54,20 @@ def test_build_many_geometries(gpu_ctx, flags):
     ref = O.OracleScene(sd, build_flags=flags).trace(rays)[0]
     assert len(np.unique(ref["instance_id"])) >= 8
     assert_hits_equal(gbrt.Scene(gpu_ctx, sd, build_flags=flags).trace(rays)[0], ref)
+
+
+@pytest.mark.parametrize("flags", [0, 2], ids=["width8", "width4"])
+def test_far_vertices(gpu_ctx, flags):
+    """Two triangles so far out that the surface area of the boxes around them
+    overflows: the others are found as before."""
+    from rustracer_gb300 import gbrt
+    sd = scenes.random_soup(2000, seed=61, size=0.15)
+    sd.vertices["pos"][-6:, :3] = np.float32([[2e19, 0, 0], [2e19, 1, 0], [2e19, 0, 1], [-2e19, 2e19, -2e19],
+                                              [-2e19, 2e19, -1e19], [-2e19, 1e19, -2e19]])
+    rays = scenes.random_rays(5000, seed=62)
+    ref = oracle_scene(sd).trace(rays)[0]
+    assert (ref["instance_id"] != 0xFFFFFFFF).mean() > 0.4
+    sc = gbrt.Scene(gpu_ctx, sd, build_flags=flags)
+    for width in (4 if flags else 8, 2):
+        sc.set_tuning(width)
+        assert_hits_equal(sc.trace(rays)[0], ref)
