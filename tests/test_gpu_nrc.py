@@ -318,3 +318,23 @@ def test_query_device_buffers(gpu_ctx):
     ms = c.query_device(p4.data_ptr(), len(pos), out.data_ptr())
     assert ms >= 0.0
     np.testing.assert_array_equal(out[:, :3].cpu().numpy(), y)
+
+
+@pytest.mark.parametrize("spp,bounces", [(1, 1), (4, 8)])
+@pytest.mark.parametrize("scene", ["zoo", "tori"])
+def test_render_disabled_equals_path_tracing_with_every_feature(gpu_ctx, scene, spp, bounces):
+    """As test_render_disabled_equals_path_tracing, on scenes with textures,
+    specular-glossiness, volumes, alpha tests, a sky and point lights: the cache's
+    shade kernel compiles texture samples and powers in line, the plain frame's
+    calls them, and the bits are the same."""
+    from rustracer_gb300 import gbrt, workloads, zoo
+    sd = zoo.material_zoo() if scene == "zoo" else workloads.batched_scene(3, max_tri=5000, min_tri=5000)[0]
+    sc = gbrt.Scene(gpu_ctx, sd)
+    lo, hi = workloads.world_box(sd, 2.0)
+    c = gbrt.Nrc(gpu_ctx, tuple(map(float, lo)), tuple(map(float, hi)), log2_table=15)
+    ubo = sd.ubo(160, 96, samples=spp, bounces=bounces, exposure=1.0, has_sky=scene == "zoo")
+    a1, a2 = gbrt.Accum(gpu_ctx, 160, 96), gbrt.Accum(gpu_ctx, 160, 96)
+    ref = sc.render(ubo, a1, mode=gbrt.MODE_WAVEFRONT)
+    r = c.render(sc, ubo, a2, disabled=True, train_samples=4096)
+    assert np.array_equal(r["image"], ref["image"])
+    assert np.array_equal(a1.download(), a2.download())

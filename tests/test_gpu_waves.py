@@ -77,3 +77,43 @@ def test_ray_query_forms(gpu_ctx, form, masked):
         assert_hits_equal(sc.trace(rays, flags)[0], ref)
         any_hit = sc.trace(rays, flags | 4)[0]  # GBRT_RAY_TERMINATE_ON_FIRST: some hit of the ray
         assert np.array_equal(any_hit["t"] >= 0, ref["t"] >= 0)
+
+
+@pytest.mark.parametrize("per_warp", [2, 16], ids=["two rays a warp", "full warps"])
+@pytest.mark.parametrize("off", [-2, -1, 0, 1])
+def test_ray_counts_at_launch_shapes(gpu_ctx, soup, per_warp, off):
+    """Counts where a query's launch goes from one-warp blocks to full ones (two rays
+    per resident warp) and where its warps take 32 rays at a time (sixteen), of this
+    GPU: eight blocks of four warps per SM."""
+    import torch
+    from rustracer_gb300 import gbrt
+    sd, rays, ref = soup
+    count = per_warp * 32 * torch.cuda.get_device_properties(0).multi_processor_count + off
+    assert count < len(rays)
+    sc = gbrt.Scene(gpu_ctx, sd)
+    for width in (8, 2):
+        sc.set_tuning(width)
+        assert_hits_equal(sc.trace(rays[:count])[0], ref[:count])
+        any_hits = sc.trace(rays[:count], 0x4)[0]
+        assert np.array_equal(any_hits["instance_id"] == 0xFFFFFFFF, ref[:count]["instance_id"] == 0xFFFFFFFF)
+
+
+@pytest.mark.parametrize("blocks", [7, 8])
+@pytest.mark.parametrize("off", [-1, 0, 1])
+def test_frames_at_launch_shapes(gpu_ctx, blocks, off):
+    """Frames of two paths per resident warp, at the seven blocks per SM of the opaque
+    binary form and the eight of the others: both layouts give the same sums."""
+    import torch
+    from rustracer_gb300 import gbrt
+    sd = scenes.icosphere_scene(subdiv=3)
+    sc = gbrt.Scene(gpu_ctx, sd)
+    width = 8 * blocks * torch.cuda.get_device_properties(0).multi_processor_count + off
+    ubo = sd.ubo(width, 1, samples=1, bounces=4, exposure=1.0)
+    out = []
+    for layout in (8, 2):
+        sc.set_tuning(layout)
+        acc = gbrt.Accum(gpu_ctx, width, 1)
+        sc.render(ubo, acc, mode=gbrt.MODE_WAVEFRONT)
+        out.append(acc.download())
+    assert out[0][..., :3].max() > 0
+    assert np.array_equal(out[0], out[1])
