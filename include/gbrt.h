@@ -244,9 +244,9 @@ typedef struct gbrt_stats {
     double   device_ms;       /* CUDA-event time of the device work */
     uint32_t kernel_launches;
     uint32_t device_status;   /* 0, or GBRT_STATUS_* bits reported by kernels */
-    uint64_t node_visits;     /* BVH inner nodes visited by all traversals (varies by a few
-                                 percent between runs, as lanes share long rays) */
-    uint64_t tri_tests;       /* ray-triangle tests */
+    uint64_t node_visits;     /* BVH inner nodes visited by all traversals */
+    uint64_t tri_tests;       /* ray-triangle tests; in the 8-wide layout both vary by a few
+                                 percent between runs, as lanes share long rays (no hit does) */
     double   stage_ms[4];     /* with GBRT_RENDER_STAGE_TIMING (wavefront form):
                                  extend, shade, shadow, other kernels */
 } gbrt_stats;
@@ -297,7 +297,14 @@ int gbrt_ctx_destroy(gbrt_ctx* ctx);
 /* Message of the last failed call on ctx ("" if none).  ctx may be NULL for
  * errors of gbrt_ctx_create. */
 const char* gbrt_last_error(const gbrt_ctx* ctx);
-/* Free / total device memory as seen by this context. */
+/* Free / total device memory as seen by this context.
+ *
+ * A context keeps memory between calls, until gbrt_ctx_destroy: the wave
+ * buffers and host-array staging of its largest frame and query so far, the
+ * scratch of its largest build (about 270 B per triangle; more than 1 GiB is
+ * given back when the build ends, everything when it fails) and, from the
+ * first gbrt_job_submit on, up to 256 MiB of finished jobs' frame sums and
+ * images. */
 int gbrt_ctx_mem_info(gbrt_ctx* ctx, uint64_t* free_bytes, uint64_t* total_bytes);
 /* Waits for all work queued on the context's stream; returns
  * GBRT_E_DEVICE_LIMIT if a frame queued with GBRT_RENDER_ASYNC since the
@@ -357,9 +364,10 @@ int gbrt_tlas_build(gbrt_scene* scene, const gbrt_instance* instances, uint32_t 
  * the TLAS, the same identity / non-identity class), the update is
  * incremental: transformed instances merged into the world BVH re-transform
  * their triangles and both layouts of the world BVH are refit in place (a
- * full build once the wide one's SAH cost proxy has drifted 1.3x); a TLAS is rebuilt over the instances' new world
- * boxes with the BLASes untouched.  Any other change takes a full build, as
- * gbrt_tlas_build.  Hits are the same as after gbrt_tlas_build with these
+ * full build once the wide one's SAH cost proxy has drifted 1.3x; both share
+ * one clustering, so the binary one drifts with it); a TLAS is rebuilt over
+ * the instances' new world boxes with the BLASes untouched.  Any other change
+ * takes a full build, as gbrt_tlas_build.  Hits are the same as after gbrt_tlas_build with these
  * instances.  GBRT_E_BUSY while the context has unfinished jobs.
  * Synchronous. */
 int gbrt_tlas_update(gbrt_scene* scene, const gbrt_instance* instances, uint32_t n);
@@ -554,7 +562,7 @@ int gbrt_scene_set_tuning(gbrt_scene* scene, uint32_t width, uint32_t sort_rays)
  * to 2^26 paths instead of 2^24, and a job of at least 2^24 paths runs alone
  * through the single-frame kernels when its turn comes (it fills the GPU by
  * itself).  Set it before the context's first submit: the wave buffers
- * (216 B per path) are sized then. */
+ * (264 B per path) are sized then. */
 #define GBRT_JOB_LARGE_WAVES 0x100u
 
 typedef struct gbrt_job_desc {

@@ -111,9 +111,10 @@ GB_D void nrc_encode_h(const NrcView& v, float3 p, float (&x)[kNrcIn]) {
     }
 }
 
-// Table reads of a query: levels that fit the first-level cache (the coarsest
-// three: 23, 63 and 171 KB at base 16 and growth 1.447) go through it, the
-// others, which never hit there, straight to the second.
+// Table reads of a query: the coarsest three levels go through the first-level
+// cache, the others straight to the second.  Three is chosen for the default
+// resolutions (base 16, growth 1.447: 23, 63 and 171 KB; five measured the same);
+// with others it is as correct and may not be the best.
 constexpr int kCachedLevels = 3;
 GB_D uint4 table_quad(const __half2* grid, uint32_t i, bool cached) {  // entries 4 i .. 4 i + 3
     const uint4* p = reinterpret_cast<const uint4*>(grid) + i;

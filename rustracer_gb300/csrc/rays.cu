@@ -50,7 +50,11 @@ cudaError_t launch_trace_rays_persistent(const DevScene& s, const gbrt_ray* rays
     // the TLAS walk and the alpha test for every scene took 254 us for 1,500,001
     // random closest hits on an opaque icosphere of 327,680 triangles, its own
     // 176 (any hits 255 and 197; with alpha tests, material zoo, 367 and 266).  With
-    // 8, 7, 6 and 5 blocks per SM: 176, 183, 190 and 213.
+    // 8, 7, 6 and 5 blocks per SM: 174, 179, 188 and 205.  The forms that spill at 64
+    // registers are within 8% of their best at 8 too: closest hits in the zoo 264,
+    // 258, 271 and 300, in the binary layout 413, 397, 400 and 418 (zoo 479, 488, 465,
+    // 488), under the TLAS of instanced tori 674, 653, 669 and 695, of a city 421,
+    // 405, 397 and 420.
     using Kernel = void (*)(DevScene, const gbrt_ray*, uint32_t, uint32_t, gbrt_hit*, uint32_t*, DeviceCounters*);
     static constexpr Kernel kernels[2][6] = {
         {trace_rays_persistent<false, 0>, trace_rays_persistent<false, 1>, trace_rays_persistent<false, 2>,

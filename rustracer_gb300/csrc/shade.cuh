@@ -366,7 +366,8 @@ GB_D float3 offset_ray(float3 p, float3 n) {
 
 // ---------------------------------------------------------------------------
 // Texture sampling (software bilinear, no mips, Vulkan wrap rules; sRGB
-// decoded per texel through a 256-entry table computed on the host).
+// and 8-bit linear values decoded per texel through a table computed on the
+// host).
 // Arithmetic is unfused so the any-hit alpha test matches the CPU exactly.
 // ---------------------------------------------------------------------------
 // 8-bit channel values as floats: entries 0..255 sRGB-decoded, 256..511 c / 255
@@ -427,8 +428,8 @@ GB_D float4 sample_tex2d(const DevTexture& t, float u, float v) {
 // Texture samples of the full-feature shade kernels, out of line: closest_hit
 // takes up to a dozen, and inlined they made it so large that its warps waited
 // for instructions two thirds of the time (materials frame: shade 2.06 -> 1.42
-// ms).  The radiance-cache form keeps them in line, where its results are the
-// plain frame's to the bit.
+// ms).  The radiance-cache form keeps them in line; with the cache off it gives
+// the plain frame's bits on scenes of every feature.
 static __device__ __noinline__ float4 sample_tex2d_call(const void* data, uint32_t w, uint32_t h, uint32_t format,
                                                         uint32_t wrap_s, uint32_t wrap_t, float u, float v) {
     DevTexture t;

@@ -30,8 +30,8 @@
 #ifndef GBRT_TRACE_MINB
 #define GBRT_TRACE_MINB 8
 #endif
-// The opaque binary form runs at 7, where it spills little (72 registers; 72 to
-// 88 B of stores at 64): icosphere frames of 640 x 360 x 4 with 327,680 triangles
+// The opaque binary form runs at 7, where it hardly spills (72 registers, at most
+// 8 B of stores; 72 to 88 B at 64): icosphere frames of 640 x 360 x 4 with 327,680 triangles
 // 1.96 -> 1.90 ms, 20,480 1.33 -> 1.29, 24 frames of 256 x 256 x 2 6.76 -> 6.67.  With
 // the alpha test 8 are better there too: instanced tori of 1280 x 720 x 8 15.6 ms
 // at 7, 15.3 at 8.
@@ -73,7 +73,7 @@ constexpr int trace_minb(int mode) {
 
 namespace gbrt {
 
-// 2 blocks of 256: at most 128 registers, no spills.  Sweep on the icosphere
+// 2 blocks of 256: 128 registers, of which the full-feature form spills 16 B.  Sweep on the icosphere
 // frame: (256, 2) 3768 Mrays/s; (256, 3) 3677 and (128, 6) 3659 with 80
 // registers and spills; (256, 1) let ptxas take more registers, one block per
 // SM, 3010.
