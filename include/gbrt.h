@@ -543,7 +543,8 @@ int gbrt_scene_set_tuning(gbrt_scene* scene, uint32_t width, uint32_t sort_rays)
  * While a context has unfinished jobs, its synchronous calls that use the
  * stream (render, trace, builds, skinning, lights, skybox) return
  * GBRT_E_BUSY, and a scene or accumulation buffer used by an unfinished job
- * cannot be destroyed or reset.  A skinned scene is animated by jobs that
+ * cannot be destroyed or reset.  A job submitted while another thread is inside
+ * such a call starts when that call returns.  A skinned scene is animated by jobs that
  * carry skins: the scheduler admits such a job once no active job uses that
  * scene, then skins it and rebuilds its BVH before the job's first wave.
  *

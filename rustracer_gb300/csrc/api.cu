@@ -695,7 +695,8 @@ int gbrt_scene_destroy(gbrt_scene* s) {
 int gbrt_blas_build(gbrt_scene* s, const gbrt_geo_range* r, uint32_t n, uint32_t flags) {
     if (!s) return GBRT_E_INVALID;
     gbrt_ctx* c = s->ctx;
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if (n && !r) return fail(c, GBRT_E_INVALID, "ranges is NULL");
     if (flags & ~(GBRT_BUILD_NO_FLATTEN | GBRT_BUILD_WIDTH4)) return fail(c, GBRT_E_INVALID, "unknown build flags");
     s->build_flags = flags;
@@ -719,7 +720,8 @@ int gbrt_blas_build(gbrt_scene* s, const gbrt_geo_range* r, uint32_t n, uint32_t
 
 int gbrt_tlas_build(gbrt_scene* s, const gbrt_instance* in, uint32_t n) {
     if (!s) return GBRT_E_INVALID;
-    if (jobs_outstanding(s->ctx)) return fail(s->ctx, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(s->ctx);
+    if (turn.busy) return fail(s->ctx, GBRT_E_BUSY, "jobs are running on this context");
     if (n && !in) return fail(s->ctx, GBRT_E_INVALID, "instances is NULL");
     DeviceGuard g(s->ctx->device);
     s->instances.assign(in, in + n);
@@ -729,7 +731,8 @@ int gbrt_tlas_build(gbrt_scene* s, const gbrt_instance* in, uint32_t n) {
 int gbrt_tlas_update(gbrt_scene* s, const gbrt_instance* in, uint32_t n) {
     if (!s) return GBRT_E_INVALID;
     gbrt_ctx* c = s->ctx;
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if (n && !in) return fail(c, GBRT_E_INVALID, "instances is NULL");
     if (!s->built) return fail(c, GBRT_E_NOT_BUILT, "build the TLAS with gbrt_tlas_build before updating it");
     if (n != s->instances.size()) return fail(c, GBRT_E_INVALID, "instance count differs from the built TLAS");
@@ -742,14 +745,16 @@ int gbrt_skin_and_refit(gbrt_scene* s, const gbrt_skin_raw* skins, uint32_t nski
     gbrt_ctx* c = s->ctx;
     if (nskin && !skins) return fail(c, GBRT_E_INVALID, "skins is NULL");
     if (!s->built) return fail(c, GBRT_E_NOT_BUILT, "build the TLAS before skinning");
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     return skin_scene(s, skins, nskin);
 }
 
 int gbrt_lights_set(gbrt_scene* s, const gbrt_light_raw* d, uint32_t nd, const gbrt_light_raw* p, uint32_t np) {
     if (!s) return GBRT_E_INVALID;
     gbrt_ctx* c = s->ctx;
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if ((nd && !d) || (np && !p)) return fail(c, GBRT_E_INVALID, "lights pointer is NULL");
     DeviceGuard g(c->device);
     CU(c, upload(s->dlights, d, nd, c->stream), "upload(dlights)");
@@ -770,7 +775,8 @@ int gbrt_skybox_set_ex(gbrt_scene* s, uint32_t size, const void* faces, uint32_t
     gbrt_ctx* c = s->ctx;
     if (format != GBRT_TEX_RGBA8_SRGB && format != GBRT_TEX_RGBA32F)
         return fail(c, GBRT_E_INVALID, "skybox format must be GBRT_TEX_RGBA8_SRGB or GBRT_TEX_RGBA32F");
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     DeviceGuard g(c->device);
     if (!faces || size == 0) {
         s->sky.release();
@@ -845,7 +851,8 @@ int gbrt_render_ex(gbrt_scene* s, const gbrt_ubo* ubo, gbrt_accum* acc, uint8_t*
                    const gbrt_render_opts* opts) {
     if (!s) return GBRT_E_INVALID;
     gbrt_ctx* c = s->ctx;
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if (!ubo || !acc) return fail(c, GBRT_E_INVALID, "ubo or accumulation buffer is NULL");
     if (!s->built) return fail(c, GBRT_E_NOT_BUILT, "build the BLAS and TLAS before rendering");
     if (acc->ctx != c) return fail(c, GBRT_E_INVALID, "accumulation buffer belongs to another context");
@@ -936,7 +943,8 @@ int gbrt_scene_autotune(gbrt_scene* s, const gbrt_ubo* ubo, uint32_t width, uint
     gbrt_ctx* c = s->ctx;
     if (!ubo || width == 0 || height == 0) return fail(c, GBRT_E_INVALID, "NULL probe UBO or empty probe image");
     if (!s->built) return fail(c, GBRT_E_NOT_BUILT, "build the BLAS and TLAS before tuning");
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if (ubo->number_of_bounces > 31 || ubo->number_of_samples == 0)
         return fail(c, GBRT_E_INVALID, "probe needs 1..31 bounces and at least one sample");
     DeviceGuard g(c->device);
@@ -1036,7 +1044,8 @@ int gbrt_scene_set_tuning(gbrt_scene* s, uint32_t width, uint32_t sort_rays) {
     gbrt_ctx* c = s->ctx;
     if (width != 2 && width != 4 && width != 8) return fail(c, GBRT_E_INVALID, "width must be 2, 4 or 8");
     if (!s->built) return fail(c, GBRT_E_NOT_BUILT, "build the BLAS and TLAS before tuning");
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     DeviceGuard g(c->device);
     if (width != 2 && (uint32_t)cw_width(s) != width) {
         s->build_flags ^= GBRT_BUILD_WIDTH4;
@@ -1057,7 +1066,8 @@ int gbrt_trace_rays_device(gbrt_scene* s, const gbrt_ray* d_rays, uint32_t n, ui
     gbrt_ctx* c = s->ctx;
     if (n && (!d_rays || !d_hits)) return fail(c, GBRT_E_INVALID, "rays or hits is NULL");
     if (!s->built) return fail(c, GBRT_E_NOT_BUILT, "build the BLAS and TLAS before tracing");
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     DeviceGuard g(c->device);
     CU(c, launch_trace_rays_persistent(s->view, d_rays, n, flags, d_hits, c->trace_work.as<uint32_t>(), nullptr,
                                        c->stream),
@@ -1069,7 +1079,8 @@ int gbrt_trace_rays(gbrt_scene* s, const gbrt_ray* rays, uint32_t n, uint32_t fl
                     gbrt_stats* stats) {
     if (!s) return GBRT_E_INVALID;
     gbrt_ctx* c = s->ctx;
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if (n && (!rays || !hits)) return fail(c, GBRT_E_INVALID, "rays or hits is NULL");
     if (!s->built) return fail(c, GBRT_E_NOT_BUILT, "build the BLAS and TLAS before tracing");
     DeviceGuard g(c->device);
@@ -1187,7 +1198,8 @@ extern "C" int gbrt_scene_rebuild_noalloc(gbrt_scene* s, const gbrt_vertex* d_ve
     if (!s) return GBRT_E_INVALID;
     gbrt_ctx* c = s->ctx;
     // queued jobs read this scene's BVH and host view from the job thread
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if (!s->built) return fail(c, GBRT_E_NOT_BUILT, "build the TLAS with gbrt_tlas_build before rebuilding");
     bool transformed = s->view.has_tlas;  // flattened transformed instances have no TLAS but count too
     for (const gbrt_instance& in : s->instances)

@@ -65,7 +65,10 @@ struct gbrt_ctx {
     gbrt::WfSide side;  // shadow-stage stream of single-frame renders
     StageTimer timer;
     std::mutex mu;
-    gbrt_host::JobQueue* jobs = nullptr;  // created by the first gbrt_job_submit
+    // Held by a synchronous call while it uses the stream and the buffers above (SyncCall), and by the job
+    // worker from a queue's first admission until it is idle.  Taken before a JobQueue's own mutex.
+    std::mutex exec;
+    std::atomic<gbrt_host::JobQueue*> jobs{nullptr};  // created by the first gbrt_job_submit
     uint64_t jobs_budget = 0;             // gbrt_jobs_configure before the first job
     std::atomic<uint32_t> inject_admit_oom{0};  // gbrt_jobs_inject: admissions still to fail
     uint32_t jobs_policy = 0;
@@ -176,5 +179,18 @@ gbrt_ctx* nrc_ctx(const gbrt_nrc* r);
 void jobs_shutdown(gbrt_ctx* c);
 // Jobs submitted and not yet finished on this context.
 uint32_t jobs_outstanding(const gbrt_ctx* c);
+
+// A synchronous call's turn on the context: not given while jobs are
+// outstanding (the call answers GBRT_E_BUSY); a job that another thread submits
+// during the call waits for its end.
+struct SyncCall {
+    std::unique_lock<std::mutex> hold;
+    bool busy;
+    explicit SyncCall(gbrt_ctx* c) : busy(jobs_outstanding(c) != 0) {
+        if (busy) return;
+        hold = std::unique_lock<std::mutex>(c->exec);  // the worker is about to let go, if it has it at all
+        busy = jobs_outstanding(c) != 0;
+    }
+};
 
 }  // namespace gbrt_host

@@ -475,8 +475,14 @@ void JobQueue::fail_active(int code, const std::string& msg) {
 
 void JobQueue::run() {
     cudaSetDevice(ctx->device);
+    std::unique_lock<std::mutex> turn(ctx->exec, std::defer_lock);  // on the stream, while there are jobs
     std::unique_lock<std::mutex> lk(mu);
     for (;;) {
+        if (!turn.owns_lock() && !queued.empty()) {  // a synchronous call of another thread may be running
+            lk.unlock();
+            turn.lock();
+            lk.lock();
+        }
         while (admit_one(lk)) {
         }
         // retire completed waves (in order)
@@ -495,6 +501,7 @@ void JobQueue::run() {
         }
         if (stop && queued.empty() && active.empty()) break;
         if (!queued.empty() && active.empty()) continue;  // admission retries at once
+        if (turn.owns_lock() && active.empty()) turn.unlock();
         cv_work.wait(lk);
     }
 }
@@ -569,12 +576,12 @@ int gbrt_jobs_configure(gbrt_ctx* c, uint64_t budget, uint32_t policy) {
     if (!c) return GBRT_E_INVALID;
     if ((policy & ~GBRT_JOB_LARGE_WAVES) > GBRT_JOB_POLICY_FIFO) return fail(c, GBRT_E_INVALID, "unknown job policy");
     std::lock_guard<std::mutex> lk(c->mu);
-    if (c->jobs) {
-        std::lock_guard<std::mutex> lq(c->jobs->mu);
-        if (budget) c->jobs->budget = budget;
-        c->jobs->policy = policy & ~GBRT_JOB_LARGE_WAVES;
+    if (JobQueue* q = c->jobs) {
+        std::lock_guard<std::mutex> lq(q->mu);
+        if (budget) q->budget = budget;
+        q->policy = policy & ~GBRT_JOB_LARGE_WAVES;
         // the wave buffers were sized at the first submit: larger waves only up to them
-        c->jobs->deep_cap = std::min((policy & GBRT_JOB_LARGE_WAVES) ? kWaveCapLarge : kWaveCapDeep, c->wf.cap);
+        q->deep_cap = std::min((policy & GBRT_JOB_LARGE_WAVES) ? kWaveCapLarge : kWaveCapDeep, c->wf.cap);
         return GBRT_OK;
     }
     c->jobs_budget = budget;
@@ -619,6 +626,7 @@ int gbrt_job_submit(gbrt_ctx* c, const gbrt_job_desc* d, uint64_t* job_id) {
     {
         std::lock_guard<std::mutex> lk(c->mu);
         if (!c->jobs) {
+            std::lock_guard<std::mutex> turn(c->exec);  // the wave buffers below may be another thread's in use
             DeviceGuard g(c->device);
             auto q = std::make_unique<JobQueue>();
             q->ctx = c;
@@ -644,8 +652,9 @@ int gbrt_job_submit(gbrt_ctx* c, const gbrt_job_desc* d, uint64_t* job_id) {
                 if (q->pool) cudaMemPoolDestroy(q->pool);
                 return cuda_fail(c, e, "job scheduler setup");
             }
-            c->jobs = q.release();
-            c->jobs->worker = std::thread([q = c->jobs] { q->run(); });
+            JobQueue* made = q.release();
+            c->jobs = made;
+            made->worker = std::thread([made] { made->run(); });
         }
     }
     JobQueue* q = c->jobs;
@@ -717,16 +726,18 @@ int gbrt_jobs_inject(gbrt_ctx* c, uint32_t kind, uint32_t count) {
 
 int gbrt_job_poll(gbrt_ctx* c, uint64_t id, gbrt_job_info* info) {
     if (!c) return GBRT_E_INVALID;
-    if (!c->jobs) return fail(c, GBRT_E_INVALID, "unknown job id");
-    std::unique_lock<std::mutex> lk(c->jobs->mu);
-    return job_result(c->jobs, c, id, info, lk, false, 0);
+    JobQueue* q = c->jobs;
+    if (!q) return fail(c, GBRT_E_INVALID, "unknown job id");
+    std::unique_lock<std::mutex> lk(q->mu);
+    return job_result(q, c, id, info, lk, false, 0);
 }
 
 int gbrt_job_wait(gbrt_ctx* c, uint64_t id, uint32_t timeout_ms, gbrt_job_info* info) {
     if (!c) return GBRT_E_INVALID;
-    if (!c->jobs) return fail(c, GBRT_E_INVALID, "unknown job id");
-    std::unique_lock<std::mutex> lk(c->jobs->mu);
-    return job_result(c->jobs, c, id, info, lk, true, timeout_ms);
+    JobQueue* q = c->jobs;
+    if (!q) return fail(c, GBRT_E_INVALID, "unknown job id");
+    std::unique_lock<std::mutex> lk(q->mu);
+    return job_result(q, c, id, info, lk, true, timeout_ms);
 }
 
 }  // extern "C"

@@ -982,7 +982,7 @@ __global__ void nrc_copy_kernel(const float* grid_w, uint32_t ngrid2, __half2* g
 using gbrt_host::DevBuf;
 using gbrt_host::DeviceGuard;
 using gbrt_host::fail;
-using gbrt_host::jobs_outstanding;
+using gbrt_host::SyncCall;
 
 struct gbrt_nrc {
     gbrt_ctx* ctx = nullptr;
@@ -1234,7 +1234,8 @@ int gbrt_nrc_create(gbrt_ctx* c, const gbrt_nrc_config* cfg, gbrt_nrc** out) {
 
 int gbrt_nrc_destroy(gbrt_nrc* r) {
     if (!r) return GBRT_OK;
-    if (jobs_outstanding(r->ctx)) return fail(r->ctx, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(r->ctx);
+    if (turn.busy) return fail(r->ctx, GBRT_E_BUSY, "jobs are running on this context");
     DeviceGuard g(r->ctx->device);
     cudaStreamSynchronize(r->ctx->stream);
     delete r;
@@ -1244,7 +1245,8 @@ int gbrt_nrc_destroy(gbrt_nrc* r) {
 int gbrt_nrc_params(gbrt_nrc* r, float* mlp, float* grid, int upload) {
     if (!r) return GBRT_E_INVALID;
     gbrt_ctx* c = r->ctx;
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     DeviceGuard g(c->device);
     cudaStream_t st = c->stream;
     const size_t ng = (size_t)r->nentries * 2 * 4;
@@ -1259,7 +1261,8 @@ int gbrt_nrc_params(gbrt_nrc* r, float* mlp, float* grid, int upload) {
 int gbrt_nrc_query(gbrt_nrc* r, const float* pos4, uint32_t n, float* out4) {
     if (!r) return GBRT_E_INVALID;
     gbrt_ctx* c = r->ctx;
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if (n && (!pos4 || !out4)) return fail(c, GBRT_E_INVALID, "NULL argument");
     DeviceGuard g(c->device);
     cudaStream_t st = c->stream;
@@ -1278,7 +1281,8 @@ int gbrt_nrc_query(gbrt_nrc* r, const float* pos4, uint32_t n, float* out4) {
 int gbrt_nrc_query_device(gbrt_nrc* r, const float* pos4_dev, uint32_t n, float* out4_dev, float* device_ms) {
     if (!r) return GBRT_E_INVALID;
     gbrt_ctx* c = r->ctx;
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if (n && (!pos4_dev || !out4_dev)) return fail(c, GBRT_E_INVALID, "NULL argument");
     if (((uintptr_t)pos4_dev | (uintptr_t)out4_dev) & 15u) return fail(c, GBRT_E_INVALID, "buffers must be 16-byte aligned");
     DeviceGuard g(c->device);
@@ -1299,7 +1303,8 @@ int gbrt_nrc_train(gbrt_nrc* r, const float* pos4, const float* target4, uint32_
                    float* grad_mlp, float* grad_grid) {
     if (!r) return GBRT_E_INVALID;
     gbrt_ctx* c = r->ctx;
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if (n == 0 || !pos4 || !target4) return fail(c, GBRT_E_INVALID, "empty batch or NULL argument");
     DeviceGuard g(c->device);
     cudaStream_t st = c->stream;
@@ -1403,7 +1408,8 @@ extern "C" int gbrt_render_nrc(gbrt_scene* s, gbrt_nrc* r, const gbrt_ubo* ubo, 
     if (!ubo || !acc || !opts) return fail(c, GBRT_E_INVALID, "NULL argument");
     if (r->ctx != c || acc->ctx != c) return fail(c, GBRT_E_INVALID, "cache or accumulation of another context");
     if (!s->built) return fail(c, GBRT_E_NOT_BUILT, "build the BLAS and TLAS before rendering");
-    if (jobs_outstanding(c)) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
+    SyncCall turn(c);
+    if (turn.busy) return fail(c, GBRT_E_BUSY, "jobs are running on this context");
     if (ubo->number_of_samples == 0 || ubo->total_number_of_samples < ubo->number_of_samples)
         return fail(c, GBRT_E_INVALID, "need 0 < number_of_samples <= total_number_of_samples");
     if (ubo->number_of_bounces > 31) return fail(c, GBRT_E_INVALID, "the wavefront form handles at most 31 bounces");

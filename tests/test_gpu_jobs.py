@@ -374,3 +374,52 @@ def test_builds_beside_skinned_jobs():
         assert np.array_equal(acc.download(), ref[i % 3]), i
     del sc, sc2, acc, accs
     ctx.close()
+
+
+def test_frames_beside_jobs():
+    """Frames of one thread, plain and through a radiance cache, while another submits
+    jobs: a call either has the context to itself or answers GBRT_E_BUSY, and the
+    jobs (the first one sizes the wave buffers anew) wait for it."""
+    import threading
+    from rustracer_gb300 import gbrt
+    ctx = gbrt.Context(0)
+    sds = [zoo.material_zoo(subdiv=2), scenes.icosphere_scene(subdiv=3)]
+    scs = [gbrt.Scene(ctx, sd) for sd in sds]
+    ubo = [sds[0].ubo(80, 48, samples=3, bounces=6, exposure=1.0, has_sky=True),
+           sds[1].ubo(64, 64, samples=2, bounces=5, exposure=1.0)]
+    size = [(80, 48), (64, 64)]
+    ref = [_solo(ctx, scs[k], ubo[k], *size[k])[1] for k in range(2)]
+    cache = gbrt.Nrc(ctx, (-3.0,) * 3, (3.0,) * 3, log2_table=14)
+    mine = [gbrt.Accum(ctx, *size[0]) for _ in range(2)]
+    accs = [gbrt.Accum(ctx, *size[k % 2]) for k in range(120)]
+    stop, frames, failed = threading.Event(), [0], []
+
+    def render():
+        while not stop.is_set():
+            try:
+                for a in mine:
+                    a.reset()
+                scs[0].render(ubo[0], mine[0], mode=gbrt.MODE_WAVEFRONT)
+                if not np.array_equal(mine[0].download(), ref[0]):
+                    failed.append("frame")
+                cache.render(scs[0], ubo[0], mine[1], image=False, disabled=True, train_samples=256)
+                if not np.array_equal(mine[1].download(), ref[0]):
+                    failed.append("cached frame")
+                frames[0] += 1
+            except gbrt.GbrtError as e:
+                if e.code != gbrt.E_BUSY:
+                    failed.append(e)
+
+    th = threading.Thread(target=render)
+    th.start()
+    try:
+        for k, acc in enumerate(accs):  # this thread: the job API alone
+            assert ctx.submit(scs[k % 2], ubo[k % 2], acc).wait()["status"] == 0
+    finally:
+        stop.set()
+        th.join()
+    assert not failed and frames[0] > 0, (failed[:3], frames)
+    for k, acc in enumerate(accs):
+        assert np.array_equal(acc.download(), ref[k % 2]), k
+    del scs, mine, accs, acc, cache
+    ctx.close()
