@@ -309,7 +309,7 @@ GB_D void persistent_trace_cw(const DevScene& s, uint32_t n, uint32_t* work, uin
                             oct = (d.x < 0.0f ? 1u : 0u) | (d.y < 0.0f ? 2u : 0u) | (d.z < 0.0f ? 4u : 0u);
                             sw.o[lane] = make_float4(o.x, o.y, o.z, tmin);
                             sw.s[lane] = make_float4(r.Sx, r.Sy, r.Sz, __int_as_float(r.kx | r.ky << 2 | r.kz << 4));
-                            cw_ray(r);
+                            cw_ray<!kTlas>(r);
                             sp = 0;
                             // virtual parent: one inner child (the root, node 0) in slot 0
                             ng = s.has_world ? make_uint2(0u, (1u << (24u + oct)) | 1u) : make_uint2(0u, 0u);

@@ -257,8 +257,14 @@ GB_D float2 cw_planes(uint32_t n0, uint32_t n1, uint32_t f0, uint32_t f1, int k,
 // nowhere and overflows to infinity alone); for directions below 2^-32 it is
 // infinite and the axis does not cull.  Components other than 0 keep their
 // inverse: near and far plane stay in proportion to the other axes.
+//
+// kSkip: rays without a zero component return at once, which takes the 0.4% off
+// 1.5 million closest hits that the rest costs (167.2 against 166.6 us); in the
+// TLAS forms, whose registers are short, the test spills and costs 1 to 2.5%.
 constexpr float kCwInvParallel = 7.9228162514264338e28f;
+template <bool kSkip>
 GB_D void cw_ray(TRay& r) {
+    if (kSkip && fabsf(r.d.x * r.d.y * r.d.z) > 0.0f) return;  // no zero (or NaN) among them
     // r.Sz: inverse of the largest component; its power of two
     const float most = kCwInvParallel * fmaxf(1.0f, __uint_as_float(__float_as_uint(r.Sz) & 0x7F800000u));
     auto axis = [&](float d, float inv) { return fabsf(d) > 0.0f ? inv : copysignf(most, inv); };
@@ -423,7 +429,7 @@ GB_D bool trace_tlas(const DevScene& s, const TRay& r, float3 o, float3 d, float
                         TRay orr;
                         setup_ray(orr, xform34_rn(in.inv, o, 1.0f), xform34_rn(in.inv, d, 0.0f));
                         if constexpr (kCwBlas) {
-                            cw_ray(orr);
+                            cw_ray<false>(orr);
                             if (traverse_cw<kTerminateOnFirst>(s, s.blas_cw_nodes + in.cw_node0,
                                                                s.blas_cw_tris + in.cw_tri0, orr, tmin, best,
                                                                test_alpha, ctx, st, ii))
